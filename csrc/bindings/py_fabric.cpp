@@ -49,7 +49,14 @@ std::vector<GpuDomainSpec> specs_from_topology(size_t nets_per_gpu, const std::v
       if (i >= g->domains.size()) info.name = "nvl" + std::to_string(i) + ":cuda" + std::to_string(dev);
       spec.domains.push_back(info);
     }
-    spec.pin_worker_cpu = g->cpus.size() > 1 ? g->cpus[1] : -1;
+    // Every engine of the process gets a core of its own: a worker polls without sleeping while
+    // transfers are in flight. With two engines on this GPU both workers sat on cpus[1] and took
+    // turns: four paged writes of 297 pages of 128 KiB each took 3.9 ms, the copies 80 us of them.
+    // cpus[0] is left to the caller, cpus[2] to the watcher, the last (where the all-to-all proxy
+    // runs) comes last.
+    for (size_t i = 1; i < g->cpus.size(); ++i) {
+      if (i != 2) spec.worker_cpus.push_back(g->cpus[i]);
+    }
     spec.pin_uvm_cpu = g->cpus.size() > 2 ? g->cpus[2] : -1;
     out.push_back(std::move(spec));
   }

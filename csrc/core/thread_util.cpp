@@ -3,6 +3,10 @@
 #include <pthread.h>
 #include <sched.h>
 
+#include <map>
+#include <mutex>
+#include <utility>
+
 #include "error.h"
 
 namespace pplx {
@@ -31,6 +35,39 @@ std::vector<int> current_affinity() {
 
 void set_thread_name(const std::string& name) {
   pthread_setname_np(pthread_self(), name.substr(0, 15).c_str());
+}
+
+namespace {
+std::mutex g_lease_mu;
+std::map<int, int>& leases() {
+  static auto* m = new std::map<int, int>();
+  return *m;
+}
+}  // namespace
+
+CpuLease::CpuLease(const std::vector<int>& candidates) {
+  std::lock_guard<std::mutex> lock(g_lease_mu);
+  int fewest = 0;
+  for (const int cpu : candidates) {
+    const auto it = leases().find(cpu);
+    const int n = it == leases().end() ? 0 : it->second;
+    if (cpu_ < 0 || n < fewest) {
+      cpu_ = cpu;
+      fewest = n;
+    }
+  }
+  if (cpu_ >= 0) ++leases()[cpu_];
+}
+
+CpuLease::~CpuLease() {
+  if (cpu_ < 0) return;
+  std::lock_guard<std::mutex> lock(g_lease_mu);
+  if (--leases()[cpu_] == 0) leases().erase(cpu_);
+}
+
+CpuLease& CpuLease::operator=(CpuLease&& o) noexcept {
+  std::swap(cpu_, o.cpu_);
+  return *this;
 }
 
 }  // namespace pplx

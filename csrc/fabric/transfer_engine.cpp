@@ -20,6 +20,7 @@ namespace pplx::fabric {
 struct TransferEngine::Worker {
   int device = -1;
   int pin_cpu = -1;
+  CpuLease lease;
   std::unique_ptr<DomainGroup> group;
   std::thread thread;
   std::mutex mu;
@@ -49,7 +50,8 @@ TransferEngine::TransferEngine(std::vector<GpuDomainSpec> gpus, DomainFactory fa
     PPLX_REQUIRE(worker_of_device_.count(spec.cuda_device) == 0, "device listed twice");
     auto w = std::make_unique<Worker>();
     w->device = spec.cuda_device;
-    w->pin_cpu = spec.pin_worker_cpu;
+    w->lease = CpuLease(spec.worker_cpus);
+    w->pin_cpu = w->lease.cpu() >= 0 ? w->lease.cpu() : spec.pin_worker_cpu;
     std::vector<std::unique_ptr<Domain>> domains;
     for (size_t i = 0; i < spec.domains.size(); ++i) {
       // every provider sits behind the fault-injection decorator (inert until armed)
@@ -93,7 +95,10 @@ void TransferEngine::stop() {
   }
   if (callback_thread_.joinable()) callback_thread_.join();
   // domains (sockets, streams, IPC mappings) go away with their groups
-  for (auto& w : workers_) w->group.reset();
+  for (auto& w : workers_) {
+    w->group.reset();
+    w->lease = CpuLease();
+  }
   if (watch_page_ != nullptr) {
     if (watch_page_cuda_) cudaFreeHost(watch_page_); else std::free(watch_page_);
     watch_page_ = nullptr;
@@ -638,7 +643,7 @@ Domain* TransferEngine::debug_domain(int device, size_t index) {
 
 TransferEngineBuilder& TransferEngineBuilder::add_gpu_domains(int cuda_device, std::vector<DomainInfo> domains,
                                                               int pin_worker_cpu, int pin_uvm_cpu) {
-  gpus_.push_back(GpuDomainSpec{cuda_device, std::move(domains), pin_worker_cpu, pin_uvm_cpu});
+  gpus_.push_back(GpuDomainSpec{cuda_device, std::move(domains), pin_worker_cpu, pin_uvm_cpu, {}});
   return *this;
 }
 

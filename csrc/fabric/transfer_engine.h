@@ -34,6 +34,8 @@ struct GpuDomainSpec {
   std::vector<DomainInfo> domains;
   int pin_worker_cpu = -1;
   int pin_uvm_cpu = -1;
+  // instead of pin_worker_cpu: the worker takes the least used of these while the engine runs
+  std::vector<int> worker_cpus;
 };
 
 class UvmWatcher {

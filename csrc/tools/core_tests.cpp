@@ -15,6 +15,7 @@
 #include "../a2a/a2a_context.h"
 #include "../a2a/a2a_proxy.h"
 #include "../core/error.h"
+#include "../core/thread_util.h"
 #include "../cumem/cumem.h"
 #include "../fabric/api.h"
 #include "../fabric/host_buffer.h"
@@ -119,6 +120,18 @@ void test_imm_counts() {
   map.inc(11);
   CHECK(flag == 1);
   CHECK(map.remove(9).has_value() && !map.remove(9).has_value());
+}
+
+void test_cpu_leases() {
+  CHECK(CpuLease(std::vector<int>{}).cpu() == -1);
+  CpuLease a({4, 7}), b({4, 7});
+  CHECK(a.cpu() == 4 && b.cpu() == 7);   // one each while there are enough
+  {
+    CpuLease c({4, 7}), d({7});
+    CHECK(c.cpu() == 4 && d.cpu() == 7);   // then shared evenly
+  }
+  a = CpuLease();                          // given back
+  CHECK(a.cpu() == -1 && CpuLease(std::vector<int>{4, 7}).cpu() == 4);
 }
 
 void test_sharding() {
@@ -592,6 +605,7 @@ int main() {
   test_error();
   test_defer_and_pools();
   test_imm_counts();
+  test_cpu_leases();
   test_sharding();
   test_host_buffers();
   test_addresses_and_topology_helpers();
