@@ -1,5 +1,6 @@
 #include "imm_count.h"
 
+#include <algorithm>
 #include <mutex>
 
 namespace pplx::fabric {
@@ -70,6 +71,31 @@ ImmIncResult ImmCountMap::inc(uint32_t imm, uint32_t n) {
     }
   }
   return ImmIncResult::kVacant;
+}
+
+uint32_t ImmCountMap::inc_each(uint32_t imm, uint32_t n, bool* reached) {
+  *reached = false;
+  {
+    std::shared_lock lock(mu_);
+    auto it = map_.find(imm);
+    if (it == map_.end()) return n;
+    Entry& e = it->second;
+    if (e.kind == Entry::Kind::kFree) {
+      e.counter->fetch_add(n, std::memory_order_acq_rel);
+      return 0;
+    }
+    if (e.kind == Entry::Kind::kExpected) {
+      int64_t have = e.counter->load(std::memory_order_acquire);
+      int64_t take = 0;
+      do {
+        take = std::min<int64_t>(n, std::max<int64_t>(e.expected - have, 0));
+      } while (take > 0 && !e.counter->compare_exchange_weak(have, have + take, std::memory_order_acq_rel));
+      *reached = take > 0 && have + take == e.expected;
+      return n - static_cast<uint32_t>(take);
+    }
+  }
+  for (uint32_t i = 0; i < n; ++i) inc(imm, 1);   // Flag: may pass zero on the way
+  return 0;
 }
 
 size_t ImmCountMap::size() const {

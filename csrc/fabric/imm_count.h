@@ -33,6 +33,9 @@ class ImmCountMap {
   std::optional<std::pair<uint32_t, uint32_t>> remove(uint32_t imm);
   // One arrival (or `n` coalesced arrivals) of `imm`.
   ImmIncResult inc(uint32_t imm, uint32_t n = 1);
+  // `n` arrivals of `imm`, each with the outcome it would have had alone: `*reached` says whether one
+  // of them completed an Expected count, the return value how many met no counter.
+  uint32_t inc_each(uint32_t imm, uint32_t n, bool* reached);
   size_t size() const;
 
  private:

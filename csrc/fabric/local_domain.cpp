@@ -37,6 +37,26 @@ void host_write(void* dst, const void* src, size_t n) {
     std::memcpy(dst, src, n);
   }
 }
+
+struct PageSpan {
+  uint32_t largest = 0;
+  bool consecutive = true;   // every index is one more than the one before
+};
+
+PageSpan page_span(const uint32_t* pages, size_t n) {
+  PageSpan out;
+  if (n == 0) return out;
+  const uint32_t first = pages[0];
+  uint32_t largest = 0, off = 0;
+  for (size_t i = 0; i < n; ++i) {   // branch-free: the compiler makes vectors of it
+    largest = std::max(largest, pages[i]);
+    off |= pages[i] ^ (first + static_cast<uint32_t>(i));
+  }
+  out.largest = largest;
+  // a list that wraps around 2^32 is none (its end would not be its largest)
+  out.consecutive = off == 0 && largest == first + static_cast<uint32_t>(n - 1) && largest >= first;
+  return out;
+}
 }  // namespace
 
 namespace {
@@ -155,6 +175,7 @@ LocalDomain::~LocalDomain() {
     for (auto& f : in_flight_) {
       if (f.event) cudaEventDestroy(f.event);
     }
+    for (cudaEvent_t e : idle_events_) cudaEventDestroy(e);
     for (auto& kv : remotes_) {
       if (kv.second.ipc_base != nullptr) cudaIpcCloseMemHandle(kv.second.ipc_base);
       if (kv.second.vmm_va != 0 && CuDriver::available()) {
@@ -671,7 +692,10 @@ void LocalDomain::run_write(const PendingWrite& w, RemoteRegion& rr, std::vector
   auto dst_page = [&](size_t i) { return dst_pages ? (*dst_pages)[page_begin + i] : 0u; };
   // Bounds of both sides, checked on the host before anything is enqueued: an index, stride
   // or offset that leaves a registered region would otherwise become an out-of-range device
-  // access (the RDMA providers of the reference get this check from the lkey / rkey).
+  // access (the RDMA providers of the reference get this check from the lkey / rkey). The end of
+  // a page grows with its index, so the largest index decides.
+  const PageSpan src_span = src_pages ? page_span(src_pages->data() + page_begin, num_pages) : PageSpan{};
+  const PageSpan dst_span = dst_pages ? page_span(dst_pages->data() + page_begin, num_pages) : PageSpan{};
   auto span_end = [](uint64_t page, uint64_t stride, uint64_t offset, uint64_t len, uint64_t* end) {
     unsigned __int128 e = static_cast<unsigned __int128>(page) * stride;
     e += offset;
@@ -680,9 +704,9 @@ void LocalDomain::run_write(const PendingWrite& w, RemoteRegion& rr, std::vector
     *end = static_cast<uint64_t>(e);
     return true;
   };
-  for (size_t i = 0; i < num_pages && length > 0; ++i) {
+  if (num_pages > 0 && length > 0) {
     uint64_t end = 0;
-    if (!span_end(dst_page(i), dst_stride, dst_offset, length, &end) || end > rr.len) {
+    if (!span_end(dst_span.largest, dst_stride, dst_offset, length, &end) || end > rr.len) {
       throw Error(ErrorKind::kDomain, "write past the end of the destination region");
     }
   }
@@ -709,9 +733,9 @@ void LocalDomain::run_write(const PendingWrite& w, RemoteRegion& rr, std::vector
       throw Error(ErrorKind::kDomain, "the source of a write is not inside a registered region");
     }
     const uint64_t base_off = src_base - region_ptr;
-    for (size_t i = 0; i < num_pages && length > 0; ++i) {
+    if (num_pages > 0 && length > 0) {
       uint64_t end = 0;
-      if (!span_end(src_page(i), src_stride, src_offset, length, &end) || end > region_len ||
+      if (!span_end(src_span.largest, src_stride, src_offset, length, &end) || end > region_len ||
           base_off > region_len - end) {
         throw Error(ErrorKind::kDomain, "read past the end of the source region");
       }
@@ -805,12 +829,22 @@ void LocalDomain::run_write(const PendingWrite& w, RemoteRegion& rr, std::vector
     a.length = length;
     a.num_pages = static_cast<uint32_t>(num_pages);
     a.error_flag = error_flag_dev_;
-    if (src_pages != nullptr) {
+    // The page tables in the cheapest form that holds them: none when both lists count up by one
+    // (the rows of a matrix), inside the kernel's parameters, or one copy to the device.
+    const uint32_t* host_src = nullptr;
+    const uint32_t* host_dst = nullptr;
+    if (src_pages != nullptr && src_span.consecutive && dst_span.consecutive) {
+      a.src_offset += (*src_pages)[page_begin] * src_stride;
+      a.dst_offset += (*dst_pages)[page_begin] * dst_stride;
+    } else if (src_pages != nullptr && num_pages <= kPagedCopyInlinePages) {
+      host_src = src_pages->data() + page_begin;
+      host_dst = dst_pages->data() + page_begin;
+    } else if (src_pages != nullptr) {
+      table_.assign(src_pages->begin() + page_begin, src_pages->begin() + page_end);
+      table_.insert(table_.end(), dst_pages->begin() + page_begin, dst_pages->begin() + page_end);
       uint32_t* scratch = device_scratch(2 * num_pages);
-      PPLX_CUDA_CHECK(cudaMemcpyAsync(scratch, src_pages->data() + page_begin, num_pages * sizeof(uint32_t),
-                                      cudaMemcpyHostToDevice, stream_));
-      PPLX_CUDA_CHECK(cudaMemcpyAsync(scratch + num_pages, dst_pages->data() + page_begin,
-                                      num_pages * sizeof(uint32_t), cudaMemcpyHostToDevice, stream_));
+      PPLX_CUDA_CHECK(cudaMemcpyAsync(scratch, table_.data(), table_.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
+                                      stream_));   // pageable: read before the call returns
       a.src_pages = scratch;
       a.dst_pages = scratch + num_pages;
     }
@@ -819,7 +853,7 @@ void LocalDomain::run_write(const PendingWrite& w, RemoteRegion& rr, std::vector
       const char* env = std::getenv("PPLX_COPY_CTAS");
       return env != nullptr ? std::atoi(env) : 0;
     }();
-    PPLX_CUDA_CHECK(launch_paged_copy(a, copy_ctas, stream_));
+    PPLX_CUDA_CHECK(launch_paged_copy(a, host_src, host_dst, rr.device == device_ && src_device == device_, copy_ctas, stream_));
   } else {
     // one side is host memory of this process: let the copy engine move each page
     for (size_t i = 0; i < num_pages; ++i) {
@@ -835,7 +869,12 @@ void LocalDomain::run_write(const PendingWrite& w, RemoteRegion& rr, std::vector
   f.imm = imm.value_or(0);
   f.imm_count = static_cast<uint32_t>(std::max<size_t>(num_pages, 1));
   f.error_flag = error_flag_host_;
-  PPLX_CUDA_CHECK(cudaEventCreateWithFlags(&f.event, cudaEventDisableTiming));
+  if (idle_events_.empty()) {
+    PPLX_CUDA_CHECK(cudaEventCreateWithFlags(&f.event, cudaEventDisableTiming));
+  } else {
+    f.event = idle_events_.back();
+    idle_events_.pop_back();
+  }
   PPLX_CUDA_CHECK(cudaEventRecord(f.event, stream_));
   in_flight_.push_back(std::move(f));
 }
@@ -902,7 +941,7 @@ void LocalDomain::poll_progress(std::vector<DomainCompletion>* out) {
         }
       }
     }
-    cudaEventDestroy(f.event);
+    idle_events_.push_back(f.event);
     in_flight_.pop_front();
     out->push_back(std::move(c));
   }

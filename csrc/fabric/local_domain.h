@@ -120,6 +120,8 @@ class LocalDomain : public Domain {
   std::map<std::pair<DomainAddress, MemoryRegionRemoteKey>, RemoteRegion> remotes_;
   std::map<std::pair<DomainAddress, MemoryRegionRemoteKey>, std::vector<PendingWrite>> waiting_mr_;
   std::deque<InFlight> in_flight_;
+  std::vector<cudaEvent_t> idle_events_;   // as many as were ever in flight at once
+  std::vector<uint32_t> table_;            // page tables on their way to the device
   std::deque<DomainCompletion> ready_;
 
   struct RecvCredit {

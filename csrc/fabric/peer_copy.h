@@ -23,11 +23,17 @@ struct PagedCopyArgs {
   uint32_t* error_flag;         // device word set to non-zero if a bounded wait ran out
 };
 
-// Launches the copy on `stream`. With addresses, strides and length all multiples of 16 bytes:
+// Page tables of at most this many pages can ride in the kernel's parameters (4 KiB of them).
+constexpr uint32_t kPagedCopyInlinePages = 480;
+
+// Launches the copy on `stream`. `host_src_pages` / `host_dst_pages`: page tables in host memory that
+// replace the device ones of `args` (both or neither; they are read before the call returns).
+// `local`: source and destination are memory of the same GPU. With addresses, strides and length all multiples of 16 bytes:
 // pages of up to 16 KiB (64 or more of them) are copied one warp per page on every SM, larger
-// ones through the bulk-copy (TMA) engine with a few CTAs; otherwise a byte-wise SIMT loop.
-// `max_ctas` <= 0 picks a default that saturates NVLink with a fraction of the SMs.
-cudaError_t launch_paged_copy(const PagedCopyArgs& args, int max_ctas, cudaStream_t stream);
+// ones through the bulk-copy (TMA) engine; otherwise a byte-wise SIMT loop. `max_ctas` <= 0 picks a
+// default: every SM for a local copy, a number that saturates NVLink with a fraction of the SMs else.
+cudaError_t launch_paged_copy(const PagedCopyArgs& args, const uint32_t* host_src_pages, const uint32_t* host_dst_pages,
+                              bool local, int max_ctas, cudaStream_t stream);
 
 // Loads the copy kernels on the current device (empty launches) and waits for them. Call once
 // per device at set-up time, never while a kernel that depends on a later copy is running.

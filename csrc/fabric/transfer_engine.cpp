@@ -31,6 +31,14 @@ struct TransferEngine::Worker {
 };
 
 namespace {
+constexpr std::chrono::microseconds kCallbackPoll(200);
+
+inline void cpu_relax() {
+#if defined(__x86_64__)
+  __builtin_ia32_pause();
+#endif
+}
+
 std::unique_ptr<Domain> default_factory(int device, int index, const DomainInfo& info) {
   if (info.provider != "local" && !info.provider.empty()) {
     throw Error(ErrorKind::kDomain, "no provider named '" + info.provider +
@@ -140,6 +148,7 @@ void TransferEngine::push_completion(TransferCompletionEntry e) {
   {
     std::lock_guard<std::mutex> lock(cq_mu_);
     cq_.push_back(std::move(e));
+    cq_size_.store(cq_.size(), std::memory_order_release);
   }
   cq_cv_.notify_one();
 }
@@ -216,19 +225,17 @@ void TransferEngine::worker_loop(Worker* w) {
           break;
         case GroupCompletion::Kind::kImm:
           // count on the worker thread so that counters move with minimal delay
-          for (uint32_t i = 0; i < c.imm_count; ++i) {
-            const ImmIncResult r = imm_counts_.inc(c.imm, 1);
-            if (r == ImmIncResult::kVacant) {
-              TransferCompletionEntry im{};
-              im.kind = TransferCompletionEntry::Kind::kImmData;
-              im.imm = c.imm;
-              push_completion(std::move(im));
-            } else if (r == ImmIncResult::kReached) {
-              TransferCompletionEntry im{};
+          {
+            bool reached = false;
+            const uint32_t vacant = imm_counts_.inc_each(c.imm, c.imm_count, &reached);
+            TransferCompletionEntry im{};
+            im.imm = c.imm;
+            if (reached) {
               im.kind = TransferCompletionEntry::Kind::kImmCountReached;
-              im.imm = c.imm;
-              push_completion(std::move(im));
+              push_completion(im);
             }
+            im.kind = TransferCompletionEntry::Kind::kImmData;
+            for (uint32_t i = 0; i < vacant; ++i) push_completion(im);
           }
           break;
       }
@@ -245,6 +252,13 @@ void TransferEngine::callback_loop() {
   set_thread_name("tx_engine_callback");
   for (;;) {
     TransferCompletionEntry e;
+    // Completions come in bursts, and waking a sleeping thread takes longer than a small copy: poll
+    // for a while after the last one before going to sleep.
+    const auto until = std::chrono::steady_clock::now() + kCallbackPoll;
+    while (cq_size_.load(std::memory_order_acquire) == 0 && !stopped_.load(std::memory_order_relaxed) &&
+           std::chrono::steady_clock::now() < until) {
+      for (int i = 0; i < 16; ++i) cpu_relax();
+    }
     {
       std::unique_lock<std::mutex> lock(cq_mu_);
       cq_cv_.wait_for(lock, std::chrono::milliseconds(50), [this] { return !cq_.empty() || stopped_.load(); });
@@ -254,6 +268,7 @@ void TransferEngine::callback_loop() {
       }
       e = std::move(cq_.front());
       cq_.pop_front();
+      cq_size_.store(cq_.size(), std::memory_order_release);
     }
     try {
       switch (e.kind) {

@@ -127,6 +127,7 @@ class TransferEngine {
   std::mutex cq_mu_;
   std::condition_variable cq_cv_;
   std::deque<TransferCompletionEntry> cq_;
+  std::atomic<size_t> cq_size_{0};   // of cq_, readable without the lock
   std::thread callback_thread_;
 
   std::mutex cb_mu_;

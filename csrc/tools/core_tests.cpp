@@ -122,6 +122,30 @@ void test_imm_counts() {
   CHECK(map.remove(9).has_value() && !map.remove(9).has_value());
 }
 
+void test_imm_count_batches() {
+  // a batch counts as its arrivals would one by one, around the edges of the expected count
+  for (uint32_t expected : {1u, 3u, 8u}) {
+    for (uint32_t n : {1u, 2u, 3u, 7u, 8u, 9u}) {
+      ImmCountMap one, many;
+      one.set_expected(5, expected);
+      many.set_expected(5, expected);
+      for (int round = 0; round < 4; ++round) {
+        uint32_t vacant = 0;
+        bool reached = false, got = false;
+        for (uint32_t i = 0; i < n; ++i) {
+          const ImmIncResult r = one.inc(5);
+          vacant += r == ImmIncResult::kVacant;
+          reached |= r == ImmIncResult::kReached;
+        }
+        CHECK(many.inc_each(5, n, &got) == vacant && got == reached);
+      }
+    }
+  }
+  ImmCountMap none;
+  bool got = true;
+  CHECK(none.inc_each(5, 4, &got) == 4 && !got);
+}
+
 void test_cpu_leases() {
   CHECK(CpuLease(std::vector<int>{}).cpu() == -1);
   CpuLease a({4, 7}), b({4, 7});
@@ -605,6 +629,7 @@ int main() {
   test_error();
   test_defer_and_pools();
   test_imm_counts();
+  test_imm_count_batches();
   test_cpu_leases();
   test_sharding();
   test_host_buffers();

@@ -74,6 +74,38 @@ def test_paged_kv_write_with_layer_notification(engines) -> None:
     assert int(dst[untouched].count_nonzero()) == 0
 
 
+@pytest.mark.parametrize("order", ["scattered", "consecutive", "one-side"])
+@pytest.mark.parametrize("pages,length", [
+    (1, 48 * 1024 + 16), (63, 16384), (64, 16384), (480, 16400), (481, 16400), (481, 32), (5, 1001), (2, 262144)])
+def test_paged_write_forms(engines, pages: int, length: int, order: str) -> None:
+    """Every form of the page tables (absent, in the kernel's parameters, on the device) with every
+    copy kernel, at the sizes where one takes over from the other. Bytes outside the pages stay."""
+    a, b = engines
+    dev = torch.device("cuda", 0)
+    stride, pool = length + (16 if length % 16 == 0 else 7), pages + 9
+    gen = torch.Generator().manual_seed(pages)
+    src = torch.randint(0, 256, (pool, stride), dtype=torch.uint8, generator=gen).to(dev)
+    dst = torch.full((pool, stride), 7, dtype=torch.uint8, device=dev)
+    hs, _ = a.register_tensor(src)
+    _, dd = b.register_tensor(dst)
+    counted, scattered = list(range(4, 4 + pages)), torch.randperm(pool, generator=gen)[:pages].tolist()
+    src_pages = scattered if order == "scattered" else counted
+    dst_pages = counted if order == "consecutive" else scattered
+    torch.cuda.synchronize()
+    w = Waiter()
+    a.submit_paged_writes(length, hs, PageIndices(src_pages), stride, 0, dd, PageIndices(dst_pages), stride, 0, None,
+                          w.done, w.error)
+    w.wait()
+    torch.cuda.synchronize()
+    want = torch.full_like(dst, 7)
+    want[dst_pages, :length] = src[src_pages, :length]
+    assert torch.equal(dst, want)
+    w = Waiter()   # one page too far on either side is refused on the host
+    a.submit_paged_writes(length, hs, PageIndices([0, pool]), stride, 0, dd, PageIndices([0, 1]), stride, 0, None,
+                          w.done, w.error)
+    assert w.event.wait(10) and "source region" in w.errors[0]
+
+
 def test_host_device_writes(engines) -> None:
     a, b = engines
     dev = torch.device("cuda", 0)
