@@ -4,6 +4,7 @@
 Generates a ninja file for every C++/CUDA source under ``csrc/`` and links
 
 * ``pplx_garden/_native.<abi>.so``   the Python extension (pybind11),
+* ``pplx_garden/_torch_ops.<abi>.so`` entry points that read torch tensors natively (links libtorch),
 * ``pplx_garden/libpplx_noalloc.so`` plain C entry points (when their source exists),
 * ``bin/pplx-fabric-debug`` and ``bin/pplx-unigram-encode`` command line tools, and
   ``bin/pplx-core-tests``, the native unit tests
@@ -44,14 +45,25 @@ def _pybind_include() -> str:
     return pybind11.get_include()
 
 
+def _torch_dir() -> Path:
+    import importlib.util
+
+    spec = importlib.util.find_spec("torch")   # without importing it
+    if spec is None or not spec.submodule_search_locations:
+        raise RuntimeError("torch is not installed")
+    return Path(spec.submodule_search_locations[0])
+
+
 def _sources() -> dict[str, list[Path]]:
-    groups: dict[str, list[Path]] = {"ext": [], "noalloc": [], "fabric_debug": [], "unigram_cli": [], "core_tests": []}
+    groups: dict[str, list[Path]] = {"ext": [], "torch_ops": [], "noalloc": [], "fabric_debug": [], "unigram_cli": [], "core_tests": []}
     for path in sorted(CSRC.rglob("*")):
         if path.suffix not in (".cpp", ".cu"):
             continue
         rel = path.relative_to(CSRC)
         if rel.parts[0] == "noalloc":
             groups["noalloc"].append(path)
+        elif rel.parts[0] == "torch_ops":
+            groups["torch_ops"].append(path)
         elif rel.parts[0] == "tools":
             if path.stem == "fabric_debug":
                 groups["fabric_debug"].append(path)
@@ -104,6 +116,8 @@ def write_ninja(verbose: bool, sanitize: str | None = None) -> Path:
         f"nvcc = {CUDA_HOME}/bin/nvcc",
         f"cxxflags = {' '.join(cxxflags + common_inc)}",
         f"pyflags = -I{py_inc} -I{_pybind_include()}",
+        f"torchflags = -I{py_inc} -isystem {_torch_dir()}/include",
+        f"torchlibs = -L{_torch_dir()}/lib -ltorch_python -ltorch_cpu -lc10 -lc10_cuda -Wl,-rpath,{_torch_dir()}/lib",
         f"nvflags = {' '.join(nvflags + common_inc)}",
         f"ldflags = -L{CUDA_HOME}/lib64 -lcudart_static -ldl -lrt -lpthread",
         "rule cxx",
@@ -118,6 +132,9 @@ def write_ninja(verbose: bool, sanitize: str | None = None) -> Path:
         "  description = NVCC $in",
         "rule link_shared",
         "  command = $cxx -shared -o $out $in $ldflags -Wl,--exclude-libs,ALL",
+        "  description = LINK $out",
+        "rule link_torch",
+        "  command = $cxx -shared -o $out $in $torchlibs -Wl,--exclude-libs,ALL",
         "  description = LINK $out",
         "rule link_exe",
         "  command = $cxx -o $out $in $ldflags",
@@ -159,6 +176,8 @@ def write_ninja(verbose: bool, sanitize: str | None = None) -> Path:
                 lines.append(f"build {obj}: cxx {src}")
                 if rel.parts[0] == "bindings":
                     lines.append("  extra = $pyflags")
+                elif rel.parts[0] == "torch_ops":
+                    lines.append("  extra = $torchflags")
             objs.append(str(obj))
         return objs
 
@@ -167,6 +186,11 @@ def write_ninja(verbose: bool, sanitize: str | None = None) -> Path:
     ext_out = Path("pplx_garden") / f"_native{ext_suffix}"
     lines.append(f"build {ext_out}: link_shared {' '.join(ext_objs)}")
     targets.append(str(ext_out))
+
+    torch_objs = compile_group(groups["torch_ops"], "torch_ops")
+    torch_out = Path("pplx_garden") / f"_torch_ops{ext_suffix}"
+    lines.append(f"build {torch_out}: link_torch {' '.join(torch_objs)}")
+    targets.append(str(torch_out))
 
     # Object files shared with the command line tools (everything except the bindings).
     core_objs = [o for o in ext_objs if "/bindings/" not in o]

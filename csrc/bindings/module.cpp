@@ -7,6 +7,7 @@
 #include "../core/error.h"
 #include "../core/log.h"
 #include "../core/thread_util.h"
+#include "native_api.h"
 #include "py_util.h"
 
 namespace py = pybind11;
@@ -25,18 +26,10 @@ PYBIND11_MODULE(_native, m) {
     try {
       if (p) std::rethrow_exception(p);
     } catch (const pplx::Error& e) {
-      switch (e.kind()) {
-        case pplx::ErrorKind::kInvalidArgument:
-          PyErr_SetString(PyExc_ValueError, e.what());
-          break;
-        case pplx::ErrorKind::kTimeout:
-          PyErr_SetString(PyExc_TimeoutError, e.what());
-          break;
-        default:
-          PyErr_SetString(PyExc_RuntimeError, e.what());
-      }
+      pplx_py::set_python_error(e);
     }
   });
+  m.attr("_api") = py::capsule(pplx_py::native_api(), pplx_py::kNativeApiName);
 
   m.def("cuda_driver_available", [] { return pplx::CuDriver::available(); },
         "True when libcuda.so.1 can be loaded in this process.");

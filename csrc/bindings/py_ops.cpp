@@ -7,10 +7,23 @@
 #include "../ops/grouped_gemm.h"
 #include "../ops/multimem.h"
 #include "../ops/router.h"
+#include "native_api.h"
+#include "py_util.h"
 
 namespace py = pybind11;
 using namespace pplx;
 using namespace pplx::ops;
+
+pplx_py::NativeApi* pplx_py::native_api() {
+  static NativeApi api = [] {
+    NativeApi a{};
+    a.topk_route = [](const TopkRouteParams& p, cudaStream_t stream) {
+      return call_guarded([&] { topk_route(p, stream); });
+    };
+    return a;
+  }();
+  return &api;
+}
 
 void bind_ops(py::module_& m) {
   m.def(
@@ -20,28 +33,6 @@ void bind_ops(py::module_& m) {
       },
       py::arg("mc_ptr"), py::arg("value"), py::arg("stream"),
       "Adds value to the 32-bit word at a multicast-mapped address on every bound GPU (one multimem.red).");
-  m.def(
-      "topk_route",
-      [](uint64_t logits, int64_t logits_stride, bool logits_bf16, uint64_t bias, uint64_t indices,
-         int64_t indices_stride, uint64_t weights, int64_t weights_stride, int tokens, int num_experts, int k,
-         uint64_t stream) {
-        TopkRouteParams p;
-        p.logits = reinterpret_cast<const void*>(logits);
-        p.logits_stride = logits_stride;
-        p.logits_bf16 = logits_bf16;
-        p.bias = reinterpret_cast<const float*>(bias);
-        p.indices = reinterpret_cast<uint32_t*>(indices);
-        p.indices_stride = indices_stride;
-        p.weights = reinterpret_cast<float*>(weights);
-        p.weights_stride = weights_stride;
-        p.tokens = tokens;
-        p.num_experts = num_experts;
-        p.k = k;
-        topk_route(p, reinterpret_cast<cudaStream_t>(stream));
-      },
-      py::arg("logits"), py::arg("logits_stride"), py::arg("logits_bf16"), py::arg("bias"), py::arg("indices"),
-      py::arg("indices_stride"), py::arg("weights"), py::arg("weights_stride"), py::arg("tokens"),
-      py::arg("num_experts"), py::arg("k"), py::arg("stream"));
   m.def(
       "grouped_fp8_gemm",
       [](uint64_t a, int64_t a_stride, uint64_t a_scale, int64_t a_scale_stride_row, int64_t a_scale_stride_k,

@@ -154,6 +154,14 @@ ProfilerHooks& profiler_hooks() {
 }
 }  // namespace
 
+void set_python_error(const pplx::Error& e) {
+  switch (e.kind()) {
+    case pplx::ErrorKind::kInvalidArgument: PyErr_SetString(PyExc_ValueError, e.what()); break;
+    case pplx::ErrorKind::kTimeout: PyErr_SetString(PyExc_TimeoutError, e.what()); break;
+    default: PyErr_SetString(PyExc_RuntimeError, e.what());
+  }
+}
+
 TorchProfilerGuard::TorchProfilerGuard(const char* name) {
   ProfilerHooks& h = profiler_hooks();
   if (!h.ok) return;

@@ -6,6 +6,8 @@
 #include <cstdint>
 #include <string>
 
+#include "../core/error.h"
+
 namespace pplx_py {
 
 namespace py = pybind11;
@@ -28,6 +30,25 @@ py::object device_bytes_capsule(uint64_t ptr, uint64_t nbytes, int device, py::o
 
 // torch tensor (uint8, 1-D) viewing [ptr, ptr+nbytes) on cuda:`device`.
 py::object device_bytes_tensor(uint64_t ptr, uint64_t nbytes, int device, py::object owner);
+
+// The Python exception of a pplx::Error (ValueError, TimeoutError or RuntimeError by its kind).
+void set_python_error(const pplx::Error& e);
+
+// Runs `f` for a caller that speaks the C API: false and a Python exception set if it throws.
+template <typename F>
+bool call_guarded(F&& f) {
+  try {
+    f();
+    return true;
+  } catch (const pplx::Error& e) {
+    set_python_error(e);
+  } catch (py::error_already_set& e) {
+    e.restore();
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+  }
+  return false;
+}
 
 // Scope that shows up in a torch profiler trace as a named range, opened from native code. The
 // reference does the same with at::RecordFunction (rust/torch-lib/src/torch_lib.cc:121-130); this

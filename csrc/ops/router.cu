@@ -1,8 +1,22 @@
-// Stand-alone top-k routing: one warp per token (the per-token work is in router.cuh).
+// Stand-alone top-k routing, one warp per token.
+//
+// A round of arg-max per chosen expert (router.cuh) costs two warp reductions and a pass over every
+// lane's registers: with 256 experts and k = 8 about 600 instructions a token, and the issue slots
+// are what a large batch waits for (32,768 tokens: 35 us for 17 MB of logits). Here a token takes
+// about half of that, whatever k is:
+//   1. every lane takes the maximum of its own PER_LANE keys;
+//   2. the k-th largest of these 32 maxima is a lower bound t of the k-th largest key (k lanes hold a
+//      key >= t), found by ranking the maxima against one another in shared memory;
+//   3. the keys >= t, usually k or a few more, are compacted into shared memory, one per lane;
+//   4. a candidate's rank among them is its place in the result.
+// Ties break to the lower expert index: expert = lane * PER_LANE + j in the vector layout, so the
+// index itself is part of the comparison. More than 32 candidates need many logits tied with the
+// bound; such a token takes the rounds of router.cuh.
 #include "router.h"
 
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cfloat>
 
 #include "../core/error.h"
@@ -11,15 +25,68 @@
 namespace pplx::ops {
 namespace {
 
-constexpr int kWarpsPerBlock = 8;
+constexpr int kMaxWarps = 8;
+
+struct alignas(16) WarpScratch {
+  uint32_t top[32];   // the lanes' maxima
+  uint4 cand[32];     // (key, expert, logit, -), in the end by rank
+};
+
+// One predicated 16-byte store: as an `if` around it the unrolled loop that calls this became a loop
+// over arrays in local memory.
+__device__ __forceinline__ void store_if(bool yes, uint4* at, uint32_t x, uint32_t y, float z) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.u32 p, %0, 0;\n"
+      "@p st.shared.v4.u32 [%1], {%2, %3, %4, %4};\n"
+      "}\n"
+      :
+      : "r"(static_cast<uint32_t>(yes)), "r"(static_cast<uint32_t>(__cvta_generic_to_shared(at))), "r"(x), "r"(y),
+        "r"(__float_as_uint(z))
+      : "memory");
+}
+
+// PER_LANE consecutive elements of a row as floats.
+template <int PER_LANE>
+__device__ __forceinline__ void load_run(const float* p, float (&v)[PER_LANE]) {
+  if constexpr (PER_LANE % 4 == 0) {
+    #pragma unroll
+    for (int j = 0; j < PER_LANE; j += 4) {
+      const float4 q = __ldg(reinterpret_cast<const float4*>(p + j));
+      v[j] = q.x; v[j + 1] = q.y; v[j + 2] = q.z; v[j + 3] = q.w;
+    }
+  } else {
+    const float2 q = __ldg(reinterpret_cast<const float2*>(p));
+    v[0] = q.x; v[1] = q.y;
+  }
+}
+template <int PER_LANE>
+__device__ __forceinline__ void load_run(const __nv_bfloat16* p, float (&v)[PER_LANE]) {
+  constexpr int kWords = PER_LANE / 2;
+  uint32_t w[kWords];
+  if constexpr (kWords % 4 == 0) {
+    #pragma unroll
+    for (int j = 0; j < kWords; j += 4) {
+      const uint4 q = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint32_t*>(p) + j));
+      w[j] = q.x; w[j + 1] = q.y; w[j + 2] = q.z; w[j + 3] = q.w;
+    }
+  } else if constexpr (kWords == 2) {
+    const uint2 q = __ldg(reinterpret_cast<const uint2*>(p));
+    w[0] = q.x; w[1] = q.y;
+  } else {
+    w[0] = __ldg(reinterpret_cast<const uint32_t*>(p));
+  }
+  #pragma unroll
+  for (int j = 0; j < kWords; ++j) {
+    v[2 * j] = __uint_as_float(w[j] << 16);
+    v[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
+  }
+}
 
 template <int PER_LANE>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32) topk_route_kernel(const TopkRouteParams p) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int token = blockIdx.x * kWarpsPerBlock + warp;
-  if (token >= p.tokens) return;
-  const size_t elem = p.logits_bf16 ? 2 : 4;
-  const void* row = static_cast<const char*>(p.logits) + static_cast<size_t>(token) * p.logits_stride * elem;
+__device__ __noinline__ void route_by_rounds(const TopkRouteParams& p, int token, int lane) {
+  const void* row = static_cast<const char*>(p.logits) + static_cast<int64_t>(token) * p.logits_stride * (p.logits_bf16 ? 2 : 4);
   uint32_t idx;
   float weight;
   route_token_warp<PER_LANE>(row, p.logits_bf16, p.bias, p.num_experts, p.k, &idx, &weight);
@@ -29,23 +96,140 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) topk_route_kernel(const T
   }
 }
 
+__device__ __forceinline__ float to_float(float x) { return x; }
+__device__ __forceinline__ float to_float(__nv_bfloat16 x) { return __bfloat162float(x); }
+
+// kVec: rows are 16-byte aligned and num_experts is a multiple of PER_LANE; a lane's experts are
+// consecutive and come in as vectors. Otherwise expert = j * 32 + lane, one element a load.
+template <int PER_LANE, typename T, bool kVec>
+__global__ void __launch_bounds__(kMaxWarps * 32) topk_route_kernel(const __grid_constant__ TopkRouteParams p) {
+  __shared__ WarpScratch scratch[kMaxWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warps = blockDim.x >> 5;
+  WarpScratch& ws = scratch[warp];
+  const int E = p.num_experts, k = p.k;
+  const bool mine = !kVec || lane * PER_LANE < E;   // a lane's run is all inside or all outside
+  float bias[PER_LANE];
+  #pragma unroll
+  for (int j = 0; j < PER_LANE; ++j) {
+    const int e = kVec ? lane * PER_LANE + j : j * 32 + lane;
+    bias[j] = p.bias != nullptr && e < E ? p.bias[e] : 0.f;
+  }
+  for (int token = blockIdx.x * warps + warp; token < p.tokens; token += gridDim.x * warps) {
+    const T* row = static_cast<const T*>(p.logits) + static_cast<int64_t>(token) * p.logits_stride;
+    float val[PER_LANE];
+    uint32_t key[PER_LANE];
+    if constexpr (kVec) {
+      #pragma unroll
+      for (int j = 0; j < PER_LANE; ++j) val[j] = 0.f;
+      if (mine) load_run<PER_LANE>(row + lane * PER_LANE, val);
+    } else {
+      #pragma unroll
+      for (int j = 0; j < PER_LANE; ++j) val[j] = j * 32 + lane < E ? to_float(row[j * 32 + lane]) : 0.f;
+    }
+    uint32_t best = 0;
+    #pragma unroll
+    for (int j = 0; j < PER_LANE; ++j) {
+      const bool valid = kVec ? mine : j * 32 + lane < E;
+      key[j] = valid ? route_key(val[j] + bias[j]) : 0u;
+      best = max(best, key[j]);
+    }
+    // rank of this lane's maximum among the 32 (equal ones in lane order)
+    ws.top[lane] = best;
+    __syncwarp();
+    int rank = 0;
+    #pragma unroll
+    for (int i = 0; i < 32; i += 4) {
+      const uint4 q = *reinterpret_cast<const uint4*>(&ws.top[i]);
+      const uint32_t other[4] = {q.x, q.y, q.z, q.w};
+      #pragma unroll
+      for (int c = 0; c < 4; ++c) rank += other[c] + (i + c < lane ? 1u : 0u) > best ? 1 : 0;
+    }
+    const uint32_t kth = __ballot_sync(0xffffffffu, rank == k - 1);
+    // fewer than k lanes hold a key: every key is a candidate
+    const uint32_t bound = max(__shfl_sync(0xffffffffu, best, __ffs(kth) - 1), 1u);
+    // the candidates' places in the scratch: any order will do, the index decides ties below
+    int total = 0;
+    uint32_t at[PER_LANE];
+    #pragma unroll
+    for (int j = 0; j < PER_LANE; ++j) {
+      const uint32_t lanes = __ballot_sync(0xffffffffu, key[j] >= bound);
+      at[j] = min(total + __popc(lanes & ((1u << lane) - 1u)), 31);
+      total += __popc(lanes);
+    }
+    uint32_t out_idx = 0;
+    float out_val = -FLT_MAX;
+    if (total <= 32) {
+      #pragma unroll
+      for (int j = 0; j < PER_LANE; ++j) {
+        store_if(key[j] >= bound, &ws.cand[at[j]], key[j], static_cast<uint32_t>(kVec ? lane * PER_LANE + j : j * 32 + lane),
+                 val[j]);
+      }
+      __syncwarp();
+      const uint4 me = ws.cand[lane];   // meaningful for lane < total
+      int place = 0;
+      for (int i = 0; i < total; ++i) {
+        const uint2 other = *reinterpret_cast<const uint2*>(&ws.cand[i]);
+        place += other.x > me.x || (other.x == me.x && other.y < me.y) ? 1 : 0;
+      }
+      __syncwarp();   // everybody has read: the winners go to their places
+      store_if(lane < total && place < k, &ws.cand[lane < total ? place : 0], me.x, me.y, __uint_as_float(me.z));
+      __syncwarp();
+      if (lane < k) {
+        out_idx = ws.cand[lane].y;
+        out_val = __uint_as_float(ws.cand[lane].z);
+      }
+      float weight;
+      softmax_of_chosen(out_val, k, lane, &weight);
+      if (lane < k) {
+        p.indices[token * p.indices_stride + lane] = out_idx;
+        p.weights[token * p.weights_stride + lane] = weight;
+      }
+    } else {
+      route_by_rounds<PER_LANE>(p, token, lane);
+    }
+    __syncwarp();   // the scratch is rewritten by the next token
+  }
+}
+
+template <int PER_LANE, typename T>
+void launch(const TopkRouteParams& p, int sms, cudaStream_t stream) {
+  constexpr uintptr_t kAlign = std::min<size_t>(16, PER_LANE * sizeof(T));
+  const bool vec = p.num_experts % PER_LANE == 0 && reinterpret_cast<uintptr_t>(p.logits) % kAlign == 0 &&
+                   p.logits_stride * sizeof(T) % kAlign == 0;
+  // Few tokens: one warp a block, so that they spread over the SMs. Many: whole waves of resident
+  // blocks whose warps loop, with the bias in registers.
+  const int warps = p.tokens <= sms * 4 ? 1 : kMaxWarps;
+  const int blocks = std::min((p.tokens + warps - 1) / warps, sms * (warps == 1 ? 4 : 64 / kMaxWarps));
+  if (vec) {
+    topk_route_kernel<PER_LANE, T, true><<<blocks, warps * 32, 0, stream>>>(p);
+  } else {
+    topk_route_kernel<PER_LANE, T, false><<<blocks, warps * 32, 0, stream>>>(p);
+  }
+}
+
+template <typename T>
+void launch_typed(const TopkRouteParams& p, int sms, cudaStream_t stream) {
+  const int per_lane = (p.num_experts + 31) / 32;
+  static_assert(sizeof(T) == 2 || sizeof(T) == 4, "bf16 or fp32 logits");
+  if (per_lane <= 2) launch<2, T>(p, sms, stream);
+  else if (per_lane <= 4) launch<4, T>(p, sms, stream);
+  else if (per_lane <= 8) launch<8, T>(p, sms, stream);
+  else if (per_lane <= 16) launch<16, T>(p, sms, stream);
+  else launch<32, T>(p, sms, stream);
+}
+
 }  // namespace
 
 void topk_route(const TopkRouteParams& p, cudaStream_t stream) {
   PPLX_REQUIRE(p.num_experts >= 1 && p.num_experts <= 1024, "between 1 and 1024 experts");
   PPLX_REQUIRE(p.k >= 1 && p.k <= 32 && p.k <= p.num_experts, "k must be in [1, min(32, num_experts)]");
   if (p.tokens == 0) return;
-  const int blocks = (p.tokens + kWarpsPerBlock - 1) / kWarpsPerBlock;
-  const int per_lane = (p.num_experts + 31) / 32;
-  if (per_lane <= 4) {
-    topk_route_kernel<4><<<blocks, kWarpsPerBlock * 32, 0, stream>>>(p);
-  } else if (per_lane <= 8) {
-    topk_route_kernel<8><<<blocks, kWarpsPerBlock * 32, 0, stream>>>(p);
-  } else if (per_lane <= 16) {
-    topk_route_kernel<16><<<blocks, kWarpsPerBlock * 32, 0, stream>>>(p);
-  } else {
-    topk_route_kernel<32><<<blocks, kWarpsPerBlock * 32, 0, stream>>>(p);
-  }
+  int device = 0, sms = 0;
+  PPLX_CUDA_CHECK(cudaGetDevice(&device));
+  PPLX_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+  if (p.logits_bf16) launch_typed<__nv_bfloat16>(p, sms, stream);
+  else launch_typed<float>(p, sms, stream);
   PPLX_CUDA_CHECK(cudaGetLastError());
 }
 

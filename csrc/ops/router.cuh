@@ -1,5 +1,6 @@
-// Top-k routing of one token by one warp, shared by the stand-alone routing kernel (router.cu)
-// and by the all-to-all's dispatch, which can route a token in the team that is about to send it.
+// Top-k routing of one token by one warp without shared memory: what the all-to-all's dispatch uses
+// when it routes a token in the team that is about to send it, and what the stand-alone kernel
+// (router.cu) falls back to when a token's logits tie too often for its own way.
 //
 // Each lane keeps PER_LANE logits in registers (expert = j * 32 + lane, so the loads of a warp
 // are coalesced). The choice is made on logit + bias, mapped to an unsigned key of the same
@@ -17,6 +18,24 @@
 
 namespace pplx::ops {
 
+// logit + bias as an unsigned of the same order; at least 1, so that 0 can mean "no candidate".
+__device__ __forceinline__ uint32_t route_key(float choice) {
+  const uint32_t bits = __float_as_uint(choice + 0.0f);   // + 0: -0 and +0 compare equal
+  return max(bits ^ ((bits >> 31) != 0 ? 0xffffffffu : 0x80000000u), 1u);
+}
+
+// Softmax over the k chosen logits; lane r < k holds the r-th, the others hold -FLT_MAX and get 0.
+__device__ __forceinline__ void softmax_of_chosen(float my_val, int k, int lane, float* weight) {
+  float m = my_val;
+  #pragma unroll
+  for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+  const float ex = lane < k ? __expf(my_val - m) : 0.f;
+  float sum = ex;
+  #pragma unroll
+  for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+  *weight = lane < k ? ex / sum : 0.f;
+}
+
 // All 32 lanes call. On return lane r < k holds the r-th chosen expert in *idx and its softmax
 // weight in *weight; the other lanes hold (0, 0).
 template <int PER_LANE>
@@ -33,10 +52,7 @@ __device__ __forceinline__ void route_token_warp(const void* logits_row, bool lo
     if (e < num_experts) {
       v = logits_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(logits_row)[e])
                       : static_cast<const float*>(logits_row)[e];
-      const float choice = (bias != nullptr ? v + bias[e] : v) + 0.0f;   // + 0: -0 and +0 compare equal
-      const uint32_t bits = __float_as_uint(choice);
-      u = bits ^ ((bits >> 31) != 0 ? 0xffffffffu : 0x80000000u);       // monotone in the float order
-      u = max(u, 1u);
+      u = route_key(bias != nullptr ? v + bias[e] : v);
     }
     val[j] = v;
     key[j] = u;
@@ -75,16 +91,8 @@ __device__ __forceinline__ void route_token_warp(const void* logits_row, bool lo
     }
   }
 
-  // softmax over the k chosen logits (lanes >= k hold -FLT_MAX and contribute exp() = 0)
-  float m = my_val;
-  #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
-  const float ex = lane < k ? __expf(my_val - m) : 0.f;
-  float sum = ex;
-  #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+  softmax_of_chosen(my_val, k, lane, weight);
   *idx = lane < k ? my_idx : 0u;
-  *weight = lane < k ? ex / sum : 0.f;
 }
 
 }  // namespace pplx::ops

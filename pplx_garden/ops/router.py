@@ -9,7 +9,7 @@ from typing import Optional
 
 import torch
 
-from pplx_garden import _native
+from pplx_garden import _torch_ops
 
 
 def topk_route_reference(logits: torch.Tensor, topk: int,
@@ -28,6 +28,10 @@ def topk_route(logits: torch.Tensor, topk: int, bias: Optional[torch.Tensor] = N
     """logits [tokens, experts] fp32 or bf16 on a CUDA device; optional bias [experts] fp32 that
     shifts the choice but not the weights. Returns (indices uint32 [tokens, k], weights fp32
     [tokens, k]), sorted by decreasing logit; ties go to the lower expert index."""
+    routed = _torch_ops.topk_route(logits, topk, bias, out_indices, out_weights)
+    if routed is not None:
+        return routed
+    # refused: say why
     if not logits.is_cuda:
         raise RuntimeError("topk_route runs on a CUDA device; use topk_route_reference on the CPU")
     assert logits.dim() == 2 and logits.stride(1) == 1
@@ -35,15 +39,6 @@ def topk_route(logits: torch.Tensor, topk: int, bias: Optional[torch.Tensor] = N
     tokens, experts = logits.shape
     if bias is not None:
         assert bias.shape == (experts,) and bias.dtype == torch.float32 and bias.is_contiguous()
-    if out_indices is None:
-        out_indices = torch.empty((tokens, topk), dtype=torch.int32, device=logits.device).view(torch.uint32)
-    if out_weights is None:
-        out_weights = torch.empty((tokens, topk), dtype=torch.float32, device=logits.device)
-    assert out_indices.shape == (tokens, topk) and out_indices.dtype == torch.uint32 and out_indices.stride(1) == 1
-    assert out_weights.shape == (tokens, topk) and out_weights.dtype == torch.float32 and out_weights.stride(1) == 1
-    _native.topk_route(
-        logits.data_ptr(), logits.stride(0), logits.dtype == torch.bfloat16,
-        0 if bias is None else bias.data_ptr(), out_indices.data_ptr(), out_indices.stride(0),
-        out_weights.data_ptr(), out_weights.stride(0), tokens, experts, topk,
-        torch.cuda.current_stream().cuda_stream)
-    return out_indices, out_weights
+    for out, dtype in ((out_indices, torch.uint32), (out_weights, torch.float32)):
+        assert out is None or (out.shape == (tokens, topk) and out.dtype == dtype and out.stride(1) == 1)
+    raise AssertionError("topk_route: unsupported arguments")

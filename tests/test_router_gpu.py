@@ -51,3 +51,27 @@ def test_ties_go_to_the_lower_index():
     idx, w = topk_route(logits, 4)
     assert idx.view(torch.int32).cpu().tolist() == [[0, 1, 2, 3]] * 3
     assert torch.allclose(w.cpu(), torch.full((3, 4), 0.25))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("experts,k,levels", [
+    (8, 8, 3), (31, 5, 4), (64, 6, 1000), (96, 8, 7), (160, 6, 50), (256, 8, 1000), (256, 8, 9), (256, 32, 40),
+    (512, 10, 2), (1000, 32, 300), (1024, 1, 5)])
+def test_ties_and_row_layouts(experts, k, levels, dtype):
+    """Few distinct logits, so that the k-th ties with many others (more than a warp's worth too), on
+    rows that can and cannot be read as vectors; the order is the stable one."""
+    dev = torch.device("cuda", 0)
+    gen = torch.Generator(device="cpu").manual_seed(experts * k + levels)
+    for tokens, row in ((1, experts), (700, experts), (9, experts + 1)):
+        # whole and half numbers up to 128: exact in bf16
+        wide = (torch.randint(0, levels, (tokens, row), generator=gen) % 256 / 2 - 50).to(dtype).to(dev)
+        logits = wide[:, :experts]
+        for bias in (None, (torch.randint(0, 3, (experts,), generator=gen) / 2).to(dev)):
+            idx, w = topk_route(logits, k, bias)
+            x = logits.float().cpu()
+            want = torch.sort(x if bias is None else x + bias.cpu(), dim=-1, descending=True, stable=True).indices[:, :k]
+            assert torch.equal(idx.view(torch.int32).cpu().long(), want)
+            # __expf is good to 2 ulp + |x| ulp; differences of logits here are below 200, and what is
+            # that far down has no weight
+            assert torch.allclose(w.cpu(), torch.softmax(torch.gather(x, 1, want), dim=-1), rtol=1e-4, atol=1e-6)
