@@ -5,13 +5,14 @@
 // are what a large batch waits for (32,768 tokens: 35 us for 17 MB of logits). Here a token takes
 // about half of that, whatever k is:
 //   1. every lane takes the maximum of its own PER_LANE keys;
-//   2. the k-th largest of these 32 maxima is a lower bound t of the k-th largest key (k lanes hold a
-//      key >= t), found by ranking the maxima against one another in shared memory;
-//   3. the keys >= t, usually k or a few more, are compacted into shared memory, one per lane;
+//   2. a bound t that at least k of these 32 maxima reach, and only a few more, is found by bisection
+//      (a comparison, a ballot and a count a step); the k-th largest key is no smaller;
+//   3. the keys >= t, usually k and a few more, are compacted into shared memory, one per lane;
 //   4. a candidate's rank among them is its place in the result.
-// Ties break to the lower expert index: expert = lane * PER_LANE + j in the vector layout, so the
-// index itself is part of the comparison. More than 32 candidates need many logits tied with the
-// bound; such a token takes the rounds of router.cuh.
+// Ties break to the lower expert index, which is part of the comparison. More than 32 candidates need
+// many logits tied with the bound; such a token takes the rounds of router.cuh.
+// Ranking the maxima against one another instead of the bisection, and carrying the logits along
+// instead of reading the k chosen ones again, took 655 instructions a token and 26.6 us.
 #include "router.h"
 
 #include <cuda_bf16.h>
@@ -26,24 +27,25 @@ namespace pplx::ops {
 namespace {
 
 constexpr int kMaxWarps = 8;
+// resident blocks of kMaxWarps warps: what the registers allow
+template <int PER_LANE> constexpr int kBlocksPerSm = PER_LANE <= 4 ? 8 : PER_LANE <= 8 ? 5 : 2;
 
 struct alignas(16) WarpScratch {
-  uint32_t top[32];   // the lanes' maxima
-  uint4 cand[32];     // (key, expert, logit, -), in the end by rank
+  uint64_t cand[32];   // key in the high word, ~expert in the low one: larger is better, 0 is none
+  uint32_t chosen[32];
 };
 
-// One predicated 16-byte store: as an `if` around it the unrolled loop that calls this became a loop
-// over arrays in local memory.
-__device__ __forceinline__ void store_if(bool yes, uint4* at, uint32_t x, uint32_t y, float z) {
+// Stores `value` where key >= bound. One predicated instruction: as an `if` around the store the
+// unrolled loop that calls this became a loop over arrays in local memory.
+__device__ __forceinline__ void store_candidate(uint32_t key, uint32_t bound, uint64_t* at, uint32_t not_expert) {
   asm volatile(
       "{\n"
       ".reg .pred p;\n"
-      "setp.ne.u32 p, %0, 0;\n"
-      "@p st.shared.v4.u32 [%1], {%2, %3, %4, %4};\n"
+      "setp.ge.u32 p, %0, %1;\n"
+      "@p st.shared.v2.u32 [%2], {%3, %0};\n"
       "}\n"
       :
-      : "r"(static_cast<uint32_t>(yes)), "r"(static_cast<uint32_t>(__cvta_generic_to_shared(at))), "r"(x), "r"(y),
-        "r"(__float_as_uint(z))
+      : "r"(key), "r"(bound), "r"(static_cast<uint32_t>(__cvta_generic_to_shared(at))), "r"(not_expert)
       : "memory");
 }
 
@@ -102,85 +104,98 @@ __device__ __forceinline__ float to_float(__nv_bfloat16 x) { return __bfloat162f
 // kVec: rows are 16-byte aligned and num_experts is a multiple of PER_LANE; a lane's experts are
 // consecutive and come in as vectors. Otherwise expert = j * 32 + lane, one element a load.
 template <int PER_LANE, typename T, bool kVec>
-__global__ void __launch_bounds__(kMaxWarps * 32) topk_route_kernel(const __grid_constant__ TopkRouteParams p) {
+__global__ void __launch_bounds__(kMaxWarps * 32, kBlocksPerSm<PER_LANE>) topk_route_kernel(const __grid_constant__ TopkRouteParams p) {
   __shared__ WarpScratch scratch[kMaxWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int warps = blockDim.x >> 5;
   WarpScratch& ws = scratch[warp];
   const int E = p.num_experts, k = p.k;
+  const uint32_t below = (1u << lane) - 1u;
   const bool mine = !kVec || lane * PER_LANE < E;   // a lane's run is all inside or all outside
   float bias[PER_LANE];
   #pragma unroll
   for (int j = 0; j < PER_LANE; ++j) {
     const int e = kVec ? lane * PER_LANE + j : j * 32 + lane;
-    bias[j] = p.bias != nullptr && e < E ? p.bias[e] : 0.f;
+    // never -0: the sum below is then never -0 either, which would not compare equal to +0 as a key
+    bias[j] = p.bias != nullptr && e < E ? p.bias[e] + 0.f : 0.f;
   }
+  int span = 1;   // lanes of the softmax
+  while (span < k) span <<= 1;
   for (int token = blockIdx.x * warps + warp; token < p.tokens; token += gridDim.x * warps) {
     const T* row = static_cast<const T*>(p.logits) + static_cast<int64_t>(token) * p.logits_stride;
-    float val[PER_LANE];
     uint32_t key[PER_LANE];
+    #pragma unroll
+    for (int j = 0; j < PER_LANE; ++j) key[j] = 0;
     if constexpr (kVec) {
-      #pragma unroll
-      for (int j = 0; j < PER_LANE; ++j) val[j] = 0.f;
-      if (mine) load_run<PER_LANE>(row + lane * PER_LANE, val);
+      if (mine) {
+        float val[PER_LANE];
+        load_run<PER_LANE>(row + lane * PER_LANE, val);
+        #pragma unroll
+        for (int j = 0; j < PER_LANE; ++j) key[j] = route_key_of_sum(val[j] + bias[j]);
+      }
     } else {
       #pragma unroll
-      for (int j = 0; j < PER_LANE; ++j) val[j] = j * 32 + lane < E ? to_float(row[j * 32 + lane]) : 0.f;
+      for (int j = 0; j < PER_LANE; ++j) {
+        if (j * 32 + lane < E) key[j] = route_key_of_sum(to_float(row[j * 32 + lane]) + bias[j]);
+      }
     }
     uint32_t best = 0;
     #pragma unroll
-    for (int j = 0; j < PER_LANE; ++j) {
-      const bool valid = kVec ? mine : j * 32 + lane < E;
-      key[j] = valid ? route_key(val[j] + bias[j]) : 0u;
-      best = max(best, key[j]);
+    for (int j = 0; j < PER_LANE; ++j) best = max(best, key[j]);
+    ws.cand[lane] = 0;
+    // at least k lanes have best >= lo, fewer than k have best >= hi; 0: fewer than k lanes hold a key
+    uint32_t lo = __reduce_min_sync(0xffffffffu, best), hi = __reduce_max_sync(0xffffffffu, best);
+    if (lo != 0) {
+      int have = 32;
+      for (int step = 0; step < 12 && have > k + 2 && hi - lo > 1; ++step) {
+        const uint32_t mid = lo + (hi - lo) / 2;
+        const int n = __popc(__ballot_sync(0xffffffffu, best >= mid));
+        if (n >= k) {
+          lo = mid;
+          have = n;
+        } else {
+          hi = mid;
+        }
+      }
     }
-    // rank of this lane's maximum among the 32 (equal ones in lane order)
-    ws.top[lane] = best;
-    __syncwarp();
-    int rank = 0;
-    #pragma unroll
-    for (int i = 0; i < 32; i += 4) {
-      const uint4 q = *reinterpret_cast<const uint4*>(&ws.top[i]);
-      const uint32_t other[4] = {q.x, q.y, q.z, q.w};
-      #pragma unroll
-      for (int c = 0; c < 4; ++c) rank += other[c] + (i + c < lane ? 1u : 0u) > best ? 1 : 0;
-    }
-    const uint32_t kth = __ballot_sync(0xffffffffu, rank == k - 1);
-    // fewer than k lanes hold a key: every key is a candidate
-    const uint32_t bound = max(__shfl_sync(0xffffffffu, best, __ffs(kth) - 1), 1u);
-    // the candidates' places in the scratch: any order will do, the index decides ties below
+    const uint32_t bound = max(lo, 1u);
+    // the candidates' places in the scratch: any order will do
+    uint32_t lanes[PER_LANE];
     int total = 0;
-    uint32_t at[PER_LANE];
     #pragma unroll
     for (int j = 0; j < PER_LANE; ++j) {
-      const uint32_t lanes = __ballot_sync(0xffffffffu, key[j] >= bound);
-      at[j] = min(total + __popc(lanes & ((1u << lane) - 1u)), 31);
-      total += __popc(lanes);
+      lanes[j] = __ballot_sync(0xffffffffu, key[j] >= bound);
+      total += __popc(lanes[j]);
     }
-    uint32_t out_idx = 0;
-    float out_val = -FLT_MAX;
     if (total <= 32) {
+      int before = 0;
       #pragma unroll
       for (int j = 0; j < PER_LANE; ++j) {
-        store_if(key[j] >= bound, &ws.cand[at[j]], key[j], static_cast<uint32_t>(kVec ? lane * PER_LANE + j : j * 32 + lane),
-                 val[j]);
+        store_candidate(key[j], bound, &ws.cand[before + __popc(lanes[j] & below)],
+                        ~static_cast<uint32_t>(kVec ? lane * PER_LANE + j : j * 32 + lane));
+        before += __popc(lanes[j]);
       }
       __syncwarp();
-      const uint4 me = ws.cand[lane];   // meaningful for lane < total
+      const uint64_t me = ws.cand[lane];
       int place = 0;
-      for (int i = 0; i < total; ++i) {
-        const uint2 other = *reinterpret_cast<const uint2*>(&ws.cand[i]);
-        place += other.x > me.x || (other.x == me.x && other.y < me.y) ? 1 : 0;
+      #pragma unroll 1
+      for (int i = 0; i < total; i += 4) {   // what is past the last candidate is 0
+        const ulonglong2 c01 = *reinterpret_cast<const ulonglong2*>(&ws.cand[i]);
+        const ulonglong2 c23 = *reinterpret_cast<const ulonglong2*>(&ws.cand[i + 2]);
+        place += c01.x > me ? 1 : 0;
+        place += c01.y > me ? 1 : 0;
+        place += c23.x > me ? 1 : 0;
+        place += c23.y > me ? 1 : 0;
       }
-      __syncwarp();   // everybody has read: the winners go to their places
-      store_if(lane < total && place < k, &ws.cand[lane < total ? place : 0], me.x, me.y, __uint_as_float(me.z));
+      if (lane < total && place < k) ws.chosen[place] = ~static_cast<uint32_t>(me);
       __syncwarp();
+      uint32_t out_idx = 0;
+      float out_val = -FLT_MAX;
       if (lane < k) {
-        out_idx = ws.cand[lane].y;
-        out_val = __uint_as_float(ws.cand[lane].z);
+        out_idx = ws.chosen[lane];
+        out_val = to_float(row[out_idx]);
       }
-      float weight;
-      softmax_of_chosen(out_val, k, lane, &weight);
+      const float weight = softmax_of_chosen(out_val, k, lane, span);
       if (lane < k) {
         p.indices[token * p.indices_stride + lane] = out_idx;
         p.weights[token * p.weights_stride + lane] = weight;
@@ -197,10 +212,10 @@ void launch(const TopkRouteParams& p, int sms, cudaStream_t stream) {
   constexpr uintptr_t kAlign = std::min<size_t>(16, PER_LANE * sizeof(T));
   const bool vec = p.num_experts % PER_LANE == 0 && reinterpret_cast<uintptr_t>(p.logits) % kAlign == 0 &&
                    p.logits_stride * sizeof(T) % kAlign == 0;
-  // Few tokens: one warp a block, so that they spread over the SMs. Many: whole waves of resident
-  // blocks whose warps loop, with the bias in registers.
+  // Few tokens: one warp a block, so that they spread over the SMs. Many: one wave of resident blocks
+  // whose warps loop, with the bias in registers.
   const int warps = p.tokens <= sms * 4 ? 1 : kMaxWarps;
-  const int blocks = std::min((p.tokens + warps - 1) / warps, sms * (warps == 1 ? 4 : 64 / kMaxWarps));
+  const int blocks = std::min((p.tokens + warps - 1) / warps, sms * (warps == 1 ? 4 : kBlocksPerSm<PER_LANE>));
   if (vec) {
     topk_route_kernel<PER_LANE, T, true><<<blocks, warps * 32, 0, stream>>>(p);
   } else {

@@ -18,22 +18,22 @@
 
 namespace pplx::ops {
 
-// logit + bias as an unsigned of the same order; at least 1, so that 0 can mean "no candidate".
-__device__ __forceinline__ uint32_t route_key(float choice) {
-  const uint32_t bits = __float_as_uint(choice + 0.0f);   // + 0: -0 and +0 compare equal
-  return max(bits ^ ((bits >> 31) != 0 ? 0xffffffffu : 0x80000000u), 1u);
+// A float that is not -0 as an unsigned of the same order; at least 1, so that 0 can mean "no candidate".
+__device__ __forceinline__ uint32_t route_key_of_sum(float choice) {
+  const uint32_t bits = __float_as_uint(choice);
+  return max(bits ^ (static_cast<uint32_t>(static_cast<int32_t>(bits) >> 31) | 0x80000000u), 1u);
 }
+__device__ __forceinline__ uint32_t route_key(float choice) { return route_key_of_sum(choice + 0.0f); }   // -0 -> +0
 
 // Softmax over the k chosen logits; lane r < k holds the r-th, the others hold -FLT_MAX and get 0.
-__device__ __forceinline__ void softmax_of_chosen(float my_val, int k, int lane, float* weight) {
+// `span`: a power of two >= k; lanes from there on need not be looked at.
+__device__ __forceinline__ float softmax_of_chosen(float my_val, int k, int lane, int span) {
   float m = my_val;
-  #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+  for (int off = span >> 1; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
   const float ex = lane < k ? __expf(my_val - m) : 0.f;
   float sum = ex;
-  #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-  *weight = lane < k ? ex / sum : 0.f;
+  for (int off = span >> 1; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+  return lane < k ? ex / sum : 0.f;
 }
 
 // All 32 lanes call. On return lane r < k holds the r-th chosen expert in *idx and its softmax
@@ -91,7 +91,7 @@ __device__ __forceinline__ void route_token_warp(const void* logits_row, bool lo
     }
   }
 
-  softmax_of_chosen(my_val, k, lane, weight);
+  *weight = softmax_of_chosen(my_val, k, lane, 32);
   *idx = lane < k ? my_idx : 0u;
 }
 
