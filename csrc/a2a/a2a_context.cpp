@@ -9,6 +9,7 @@
 #include "../core/error.h"
 #define PPLX_LOG_TARGET "pplx_garden::a2a"
 #include "../core/log.h"
+#include "../ops/router.h"
 #include "a2a_kernels.h"
 
 namespace pplx {
@@ -169,6 +170,7 @@ A2AContext::A2AContext(const A2AParams& params, int device, const std::vector<in
   PPLX_CUDA_CHECK(a2a_preload_kernels(cfg_));
   const char* trace_env = std::getenv("PPLX_A2A_TRACE");
   cfg_.trace = (trace_env != nullptr && std::atoi(trace_env) != 0) ? 1 : 0;
+  if (single_rank()) PPLX_CUDA_CHECK(a2a_preload_single());
   const char* team_env = std::getenv("PPLX_A2A_TEAM");
   if (team_env != nullptr) team_override_ = std::atoi(team_env);
 
@@ -208,6 +210,9 @@ A2AContext::A2AContext(const A2AParams& params, int device, const std::vector<in
     const size_t o_rec_rows = take(pre ? sizeof(uint32_t) * recs * cfg_.topk : 4);
     const size_t o_rec_w = take(pre ? sizeof(float) * recs * cfg_.topk : 4);
     const size_t o_rec_tok = take(pre ? sizeof(uint32_t) * 2 * recs : 4);
+    const size_t o_route_row =
+        take(single_rank() ? sizeof(uint32_t) * static_cast<size_t>(cfg_.max_num_tokens) * cfg_.topk : 4);
+    const size_t o_single_done = take(sizeof(uint32_t) * 2);
     const size_t o_status = take(sizeof(uint32_t) * 4);
     const size_t o_stats = take(sizeof(unsigned long long) * 8);
     const size_t o_trace = take(sizeof(unsigned long long) * kTraceSlots);
@@ -230,6 +235,8 @@ A2AContext::A2AContext(const A2AParams& params, int device, const std::vector<in
     st.local.rec_rows = reinterpret_cast<uint32_t*>(b + o_rec_rows);
     st.local.rec_weights = reinterpret_cast<float*>(b + o_rec_w);
     st.local.rec_token = reinterpret_cast<uint32_t*>(b + o_rec_tok);
+    st.local.route_row = reinterpret_cast<uint32_t*>(b + o_route_row);
+    st.local.single_done = reinterpret_cast<uint32_t*>(b + o_single_done);
     st.local.status = reinterpret_cast<uint32_t*>(b + o_status);
     st.local.stats = reinterpret_cast<unsigned long long*>(b + o_stats);
     st.local.trace = reinterpret_cast<unsigned long long*>(b + o_trace);
@@ -434,6 +441,29 @@ void A2AContext::dispatch(const DispatchSendArgs* send, const DispatchRecvArgs* 
     }
   }
   PPLX_CUDA_CHECK(cudaSetDevice(device_));
+  if (single_rank() && do_send && do_recv) {
+    if (send[0].logits != nullptr) {
+      ops::TopkRouteParams t;
+      t.logits = send[0].logits;
+      t.logits_stride = send[0].logits_stride;
+      t.logits_bf16 = send[0].logits_bf16 != 0;
+      t.bias = send[0].logits_bias;
+      t.indices = const_cast<uint32_t*>(send[0].indices);
+      t.indices_stride = static_cast<int64_t>(send[0].indices_stride);
+      t.weights = const_cast<float*>(send[0].weights);
+      t.weights_stride = static_cast<int64_t>(send[0].weights_stride);
+      t.bound = send[0].bound_m;
+      t.tokens = send[0].num_tokens;
+      t.num_experts = cfg_.num_experts;
+      t.k = cfg_.topk;
+      ops::topk_route(t, stream);
+    }
+    PPLX_CUDA_CHECK(a2a_launch_dispatch_single(cfg_, states_.r[0].local, s.r[0], r.r[0], stream));
+    single_dispatched_ = true;
+    commit_phase(kPhaseDispatchRecv);
+    return;
+  }
+  single_dispatched_ = false;
   // send: one item per token; recv: one item per (source group, token) slot
   const int64_t vectors = cfg_.d_payload_bytes / 16;
   const int send_team = do_send ? pick(last_tokens_, vectors) : 0;
@@ -470,6 +500,17 @@ void A2AContext::combine(const CombineSendArgs* send, const CombineRecvArgs* rec
   PPLX_REQUIRE(y_size == cfg_.out_elemsize,
                "combine: expert_y element size differs from the context's out dtype");
   PPLX_CUDA_CHECK(cudaSetDevice(device_));
+  const bool fused = do_send && do_recv;
+  if (single_rank() && do_recv && (fused ? single_dispatched_ : external_send_)) {
+    const A2ARankState& st = states_.r[0];
+    const uint8_t* rows = fused ? s.r[0].expert_y : st.recv[0] + cfg_.off_crecv;
+    const uint32_t* arrived = reinterpret_cast<const uint32_t*>(st.sync[0]) + kFlagExternalCombine * kMaxRanks * kFlagStrideWords;
+    PPLX_CUDA_CHECK(a2a_launch_combine_single(cfg_, st.local, r.r[0], rows, fused ? s.r[0].expert_y_stride : cfg_.c_stride,
+                                              arrived, y_dtype, out_dtype, stream));
+    external_send_ = false;
+    commit_phase(kPhaseCombineRecv);
+    return;
+  }
   // send: one item per expert row (per-route) or per received record (pre-reduce);
   // recv: one item per token, whose reduction reads up to eight records per output vector.
   int send_team = 0, recv_team = 0;
@@ -560,6 +601,9 @@ std::array<uint64_t, 8> A2AContext::stats(int i) const {
 std::array<uint32_t, 2> A2AContext::iterations(int i) const {
   std::array<uint32_t, 2> out{};
   PPLX_CUDA_CHECK(cudaMemcpy(out.data(), iters_ptrs_.at(i), sizeof(uint32_t) * 2, cudaMemcpyDeviceToHost));
+  std::array<uint32_t, 2> single{};
+  PPLX_CUDA_CHECK(cudaMemcpy(single.data(), states_.r[i].local.single_done, sizeof(uint32_t) * 2, cudaMemcpyDeviceToHost));
+  for (int p = 0; p < 2; ++p) out[p] += single[p];
   return out;
 }
 

@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "a2a_proxy.h"
+#include "a2a_kernels.h"
 #include "a2a_types.h"
 
 namespace pplx {
@@ -126,6 +127,10 @@ class A2AContext {
   void debug_set_next_phase(int phase) { next_phase_ = phase; }
 
  private:
+  // A group of one rank whose protocol nobody asked to see: no peer to talk to.
+  bool single_rank() const {
+    return cfg_.world == 1 && cfg_.trace == 0 && cfg_.num_experts <= kSingleMaxExperts;
+  }
   int pick(int64_t items, int64_t vectors_per_item) const;
   void require_phase(int first) const;
   void commit_phase(int last);
@@ -145,6 +150,7 @@ class A2AContext {
   int next_phase_ = kPhaseDispatchSend;
   int64_t last_tokens_ = 0;
   int team_override_ = 0;
+  bool single_dispatched_ = false;  // the last dispatch filled the single-rank tables (a2a_single.cu)
   bool external_send_ = false;  // the pending combine's send phase was played by another kernel
   struct ProxyState {
     std::unique_ptr<A2AProxy> proxy;

@@ -35,4 +35,16 @@ cudaError_t a2a_launch_combine(const A2AConfig& cfg, const A2ARankStates& states
                                const PerRank<CombineRecvArgs>& recv, int send_team, int recv_team,
                                int y_dtype, int out_dtype, cudaStream_t stream);
 
+// A group of one rank (a2a_single.cu): both phases of a dispatch or combine in one launch that needs
+// no receive region. At most kSingleMaxExperts experts (their counters live in shared memory).
+constexpr int kSingleMaxExperts = 4096;
+cudaError_t a2a_launch_dispatch_single(const A2AConfig& cfg, const A2ALocal& ws, const DispatchSendArgs& send,
+                                       const DispatchRecvArgs& recv, cudaStream_t stream);
+// Reduces rows that dispatch_single's tables locate in expert_y, or (recv.external) rows that another
+// kernel wrote into the combine receive region and announces by raising `arrived`.
+cudaError_t a2a_launch_combine_single(const A2AConfig& cfg, const A2ALocal& ws, const CombineRecvArgs& recv,
+                                      const uint8_t* rows, uint64_t row_stride, const uint32_t* arrived, int y_dtype,
+                                      int out_dtype, cudaStream_t stream);
+cudaError_t a2a_preload_single();
+
 }  // namespace pplx

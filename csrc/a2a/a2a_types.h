@@ -176,6 +176,9 @@ struct A2ALocal {
   uint32_t* rec_rows;      // pre-reduce: [num_groups * max_num_tokens][topk] row or kNoSlot
   float* rec_weights;      // pre-reduce: same shape, routing weight
   uint32_t* rec_token;     // pre-reduce: [num_groups * max_num_tokens] token index
+  uint32_t* route_row;     // [max_num_tokens * topk] expert row of each of this rank's routes, kNoSlot = none
+                           // (written by the dispatch of a group of one rank only)
+  uint32_t* single_done;   // [2] dispatches / combines of a group of one rank (a2a_single.cu)
   uint32_t* status;        // [4]
   uint32_t* host_flag;     // pinned host word (device-mapped): failure code, readable by the
                            // host without synchronising the stream

@@ -119,9 +119,10 @@ __global__ void __launch_bounds__(kMaxWarps * 32, kBlocksPerSm<PER_LANE>) topk_r
     // never -0: the sum below is then never -0 either, which would not compare equal to +0 as a key
     bias[j] = p.bias != nullptr && e < E ? p.bias[e] + 0.f : 0.f;
   }
+  const int tokens = p.bound != nullptr ? min(p.tokens, *p.bound) : p.tokens;
   int span = 1;   // lanes of the softmax
   while (span < k) span <<= 1;
-  for (int token = blockIdx.x * warps + warp; token < p.tokens; token += gridDim.x * warps) {
+  for (int token = blockIdx.x * warps + warp; token < tokens; token += gridDim.x * warps) {
     const T* row = static_cast<const T*>(p.logits) + static_cast<int64_t>(token) * p.logits_stride;
     uint32_t key[PER_LANE];
     #pragma unroll

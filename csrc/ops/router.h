@@ -22,6 +22,7 @@ struct TopkRouteParams {
   int64_t indices_stride = 0;
   float* weights = nullptr;        // [tokens, k]
   int64_t weights_stride = 0;
+  const int32_t* bound = nullptr;  // optional device word: only this many of the tokens
   int tokens = 0;
   int num_experts = 0;             // at most 1024
   int k = 0;                       // at most 32

@@ -428,3 +428,77 @@ def test_routing_fused_into_dispatch(wire: str, experts: int, topk: int, with_bi
             assert torch.equal(out[r], out2[r]), f"rank {r}: fused routing changed the combined tokens"
     finally:
         group.destroy()
+
+
+@pytest.mark.parametrize("tokens,experts,topk,hidden,kw", [
+    (1, 256, 8, 7168, dict(in_dtype=torch.bfloat16, out_dtype=torch.bfloat16)),     # 28 blocks share the token
+    (74, 16, 2, 1024, dict(in_dtype=torch.bfloat16, out_dtype=torch.float32)),      # two blocks a token
+    (75, 5, 5, 264, dict(padding=16)),                                              # hidden not a multiple of a piece
+    (149, 60, 6, 520, dict(in_dtype=torch.float16, out_dtype=torch.float16, combine_mode="pre_reduce")),
+    (1500, 1030, 16, 128, dict(padding=4, out_dtype=torch.float16)),                # two rounds of the scan
+    (9700, 8, 1, 1024, dict(in_dtype=torch.bfloat16, out_dtype=torch.bfloat16)),    # batches of 64 tokens a block
+    (700, 32, 8, 4096, dict(in_dtype=torch.float8_e4m3fn, hidden_scale=32, out_dtype=torch.bfloat16)),
+])
+def test_single_rank(tokens: int, experts: int, topk: int, hidden: int, kw: dict) -> None:
+    """A group of one rank: straight from the tokens to the rows and back, in any order with the
+    split phases, which use the receive region; bound_m, accumulate and the iteration counts."""
+    cfg = Cfg(world=1, tokens=tokens, experts=experts, topk=topk, hidden=hidden, **kw)
+    device = torch.device("cuda", 0)
+    group = _make_group(cfg, device)
+    try:
+        bound = max(1, tokens * 2 // 3)
+        prev = [torch.randn((tokens, hidden), device=device).to(cfg.out_dtype)]
+        for it, args in enumerate([{}, dict(split=True), dict(bound=bound), {},
+                                   dict(accumulate=True, out_prev=prev), dict(split=True), {}]):
+            data = _inputs(cfg, device, seed_offset=10 * it)
+            res = _run_once(cfg, group, data, device, **args)
+            args.pop("split", None), args.pop("accumulate", None)
+            _verify(cfg, data, *res, **args)
+            if "bound" in args:
+                assert torch.count_nonzero(res[3][0][bound:]) == 0
+        assert list(group.context.iterations(0)) == [7, 7]
+        # a fused dispatch whose combine is split, and the other way round
+        d = _inputs(cfg, device)[0]
+        num, ox, os_, out = _outputs(cfg, group, device)
+        scale = [d.dp_x_scale] if cfg.hidden_scale else None
+        for fused_dispatch in (True, False):
+            for send, recv in ([(True, True)] if fused_dispatch else [(True, False), (False, True)]):
+                group.dispatch(num, ox, os_, [d.dp_x], scale, [d.indices], [d.weights], None, send, recv)
+            ys = [act(ox[0], None if os_ is None else os_[0]).to(cfg.out_dtype)]
+            out[0].zero_()
+            for send, recv in ([(True, False), (False, True)] if fused_dispatch else [(True, True)]):
+                group.combine(out, [d.indices], [d.weights], ys, None, send, recv)
+            torch.cuda.synchronize()
+            group.check()
+            _verify(cfg, [d], num, ox, os_, out)
+    finally:
+        group.destroy()
+
+
+def test_single_rank_reports_bad_input() -> None:
+    """An expert that does not exist and rows that do not fit are reported, not written."""
+    cfg = Cfg(world=1, tokens=16, experts=8, hidden=64, topk=2)
+    device = torch.device("cuda", 0)
+    for fault in ("expert", "rows"):
+        group = _make_group(cfg, device)
+        try:
+            d = _inputs(cfg, device)[0]
+            num, ox, os_, out = _outputs(cfg, group, device)
+            guard = torch.full_like(ox[0], 3.0)
+            rows = guard[:20] if fault == "rows" else guard
+            indices = d.indices.view(torch.int32).clone()
+            if fault == "expert":
+                indices[5, 1] = 8
+            group.dispatch(num, [rows], None, [d.dp_x], None, [indices.view(torch.uint32)], [d.weights])
+            torch.cuda.synchronize()
+            assert group.context.status(0)[0] == (3 if fault == "expert" else 2)
+            if fault == "rows":
+                assert (guard[20:] == 3.0).all()
+            out[0].fill_(5.0)   # a combine after a failure leaves its output alone
+            group.combine(out, [d.indices], [d.weights], [torch.zeros_like(ox[0])])
+            torch.cuda.synchronize()
+            assert (out[0] == 5.0).all()
+        except RuntimeError:
+            assert group.context.failed()   # the second call may already refuse
+        finally:
+            group.destroy()
