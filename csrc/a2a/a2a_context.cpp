@@ -5,6 +5,9 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
+#include <set>
+#include <tuple>
 
 #include "../core/error.h"
 #define PPLX_LOG_TARGET "pplx_garden::a2a"
@@ -16,6 +19,18 @@ namespace pplx {
 
 namespace {
 uint32_t round_up_u32(uint32_t a, uint32_t b) { return (a + b - 1) / b * b; }
+
+// A kernel stays loaded for the life of the process: every later context on the device finds it there.
+void preload_once(const A2AConfig& cfg, int device, bool single) {
+  static std::mutex mu;
+  static std::set<std::tuple<int, int, bool>> loaded;
+  std::lock_guard<std::mutex> lock(mu);
+  const auto key = std::make_tuple(device, cfg.wire, single);
+  if (loaded.count(key) != 0) return;
+  PPLX_CUDA_CHECK(a2a_preload_kernels(cfg));
+  if (single) PPLX_CUDA_CHECK(a2a_preload_single());
+  loaded.insert(key);
+}
 
 struct NvtxRange {
   explicit NvtxRange(const char* name) { nvtxRangePushA(name); }
@@ -167,10 +182,9 @@ A2AContext::A2AContext(const A2AParams& params, int device, const std::vector<in
                  "virtual ranks x blocks must fit the GPU at one block per SM");
   }
 
-  PPLX_CUDA_CHECK(a2a_preload_kernels(cfg_));
   const char* trace_env = std::getenv("PPLX_A2A_TRACE");
   cfg_.trace = (trace_env != nullptr && std::atoi(trace_env) != 0) ? 1 : 0;
-  if (single_rank()) PPLX_CUDA_CHECK(a2a_preload_single());
+  preload_once(cfg_, device_, single_rank());
   const char* team_env = std::getenv("PPLX_A2A_TEAM");
   if (team_env != nullptr) team_override_ = std::atoi(team_env);
 

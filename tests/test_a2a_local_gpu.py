@@ -437,6 +437,8 @@ def test_routing_fused_into_dispatch(wire: str, experts: int, topk: int, with_bi
     (149, 60, 6, 520, dict(in_dtype=torch.float16, out_dtype=torch.float16, combine_mode="pre_reduce")),
     (1500, 1030, 16, 128, dict(padding=4, out_dtype=torch.float16)),                # two rounds of the scan
     (9700, 8, 1, 1024, dict(in_dtype=torch.bfloat16, out_dtype=torch.bfloat16)),    # batches of 64 tokens a block
+    (2100, 40, 9, 1032, dict(out_dtype=torch.float32)),                             # pieces of 1536 bytes, a ragged last one
+    (8000, 6, 3, 520, dict(in_dtype=torch.bfloat16, out_dtype=torch.bfloat16, combine_mode="pre_reduce")),
     (700, 32, 8, 4096, dict(in_dtype=torch.float8_e4m3fn, hidden_scale=32, out_dtype=torch.bfloat16)),
 ])
 def test_single_rank(tokens: int, experts: int, topk: int, hidden: int, kw: dict) -> None:
