@@ -8,6 +8,7 @@
 
 #include "../a2a/a2a_context.h"
 #include "../core/error.h"
+#include "native_api.h"
 #include "py_fabric.h"
 #include "py_util.h"
 
@@ -201,6 +202,32 @@ struct PyProxyProbe {
   std::unique_ptr<A2AProxy> proxy;
 };
 
+bool pplx_py::api_a2a_dispatch(void* context, const DispatchSendArgs* send, const DispatchRecvArgs* recv,
+                               cudaStream_t stream) {
+  return call_guarded([&] {
+    PyA2A& s = *static_cast<PyA2A*>(context);
+    PPLX_REQUIRE(s.ctx != nullptr, "the all-to-all context was destroyed");
+    TorchProfilerGuard range(send != nullptr && recv != nullptr ? "a2a_dispatch"
+                             : send != nullptr                  ? "a2a_dispatch_send"
+                                                                : "a2a_dispatch_recv");
+    s.ctx->dispatch(send, recv, send != nullptr, recv != nullptr, stream);
+    s.after_launch();
+  });
+}
+
+bool pplx_py::api_a2a_combine(void* context, const CombineSendArgs* send, const CombineRecvArgs* recv, int y_dtype,
+                              cudaStream_t stream) {
+  return call_guarded([&] {
+    PyA2A& s = *static_cast<PyA2A*>(context);
+    PPLX_REQUIRE(s.ctx != nullptr, "the all-to-all context was destroyed");
+    TorchProfilerGuard range(send != nullptr && recv != nullptr ? "a2a_combine"
+                             : send != nullptr                  ? "a2a_combine_send"
+                                                                : "a2a_combine_recv");
+    s.ctx->combine(send, recv, send != nullptr, recv != nullptr, y_dtype, s.out_dtype, stream);
+    s.after_launch();
+  });
+}
+
 void bind_a2a(py::module_& m) {
   py::class_<PyProxyProbe>(m, "_A2AProxyProbe")
       .def(py::init([](const py::dict& layout_args, int rank, PyEngine& engine, const py::list& peers,
@@ -324,6 +351,8 @@ void bind_a2a(py::module_& m) {
           py::arg("wait_limit_ms") = 0, py::arg("wire") = py::none(), py::arg("node_mask") = 0,
           "Create a context. `rank` may be a list: the context then plays several ranks on one "
           "GPU and sync_ptrs / recv_ptrs hold one pointer table per local rank.")
+      .def("_handle", [](PyA2A& s) { return reinterpret_cast<uint64_t>(&s); },
+           "What the entry points that read tensors natively know this context by.")
       .def("config", [](const PyA2A& s) { return config_dict(s.ctx->config()); })
       .def("dispatch_send",
            [](PyA2A& s, int num_tokens, uint64_t x_ptr, uint64_t x_stride,

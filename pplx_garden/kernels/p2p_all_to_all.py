@@ -38,6 +38,7 @@ from typing import Optional
 
 import torch
 
+from pplx_garden import _torch_ops
 from pplx_garden.distributed import ParallelGroup
 from pplx_garden.kernels.all_to_all import AllToAllKernel
 from pplx_garden.native.cumem import (
@@ -65,13 +66,6 @@ class _RankRegions:
 class _PeerMappings:
     sync: CUMemMapping
     recv: CUMemMapping
-
-
-def _sig(t: Optional[torch.Tensor]):
-    """What the argument checks of dispatch / combine depend on."""
-    if t is None:
-        return None
-    return (t.data_ptr(), t.shape, t.stride(), t.dtype)
 
 
 def check_layout_agreement(group: ParallelGroup, rank: int, layout: dict) -> None:
@@ -278,12 +272,10 @@ class P2PAllToAll(AllToAllKernel):
             except Exception:
                 cpus = []
             self._all_to_all.enable_proxy(self._engine, proxy_peers, 0, cpus[-1] if cpus else -1)
-        self._validate_only = False
         self._num_experts = num_experts
-        self._dispatch_args: dict = {}
-        self._combine_args: dict = {}
-        self._check_every = int(os.environ.get("PPLX_A2A_CHECK_EVERY", "0"))
-        self._calls = 0
+        self._plan = _torch_ops.a2a_plan(
+            self._all_to_all._handle(), num_experts_per_token, hidden_dim, hidden_dim_scale or 0,
+            self._num_local_experts, num_experts, world_size, in_dtype, out_dtype, self._quantize_mode)
 
         # No rank may signal a peer whose flags are not zeroed yet.
         if global_group is not None:
@@ -326,122 +318,54 @@ class P2PAllToAll(AllToAllKernel):
         kernel picks each token's top-k experts on ``logits + logits_bias``, takes the softmax over
         the chosen logits, WRITES them to ``indices`` / ``weights`` (pass these to ``combine``) and
         sends by them, all in the team that moves the token."""
-        a2a = self._all_to_all
-        assert a2a is not None
+        assert self._all_to_all is not None
+        if not _torch_ops.a2a_dispatch(self._plan, out_expert_num_tokens, out_expert_x, out_expert_x_scale, dp_x,
+                                       dp_x_scale, indices, weights, bound_m, do_send, do_recv, logits, logits_bias):
+            self._reject_dispatch(out_expert_num_tokens, out_expert_x, out_expert_x_scale, dp_x, dp_x_scale, indices,
+                                  weights, bound_m, do_send, do_recv, logits, logits_bias)
+
+    def _reject_dispatch(self, out_expert_num_tokens, out_expert_x, out_expert_x_scale, dp_x, dp_x_scale, indices,
+                         weights, bound_m, do_send, do_recv, logits, logits_bias) -> None:
+        """Raises for what the native checks of ``dispatch`` refused."""
         assert do_send or do_recv
-        if logits is not None:
-            return self._dispatch_routed(out_expert_num_tokens, out_expert_x, out_expert_x_scale, dp_x,
-                                         dp_x_scale, indices, weights, bound_m, do_send, do_recv, logits,
-                                         logits_bias)
-        # A serving loop calls with the same tensors step after step: the checks below run once
-        # per distinct set of (address, shape, strides, dtype) and the packed arguments are kept.
-        key = (_sig(out_expert_num_tokens), _sig(out_expert_x), _sig(out_expert_x_scale), _sig(dp_x),
-               _sig(dp_x_scale), _sig(indices), _sig(weights), _sig(bound_m))
-        cached = self._dispatch_args.get(key)
-        if cached is not None:
-            send, recv, out_rows, quantize = cached
-            stream = torch.cuda.current_stream().cuda_stream
-            if do_send and do_recv:
-                a2a.dispatch(*send, *recv, stream, out_rows, quantize)
-            elif do_send:
-                a2a.dispatch_send(*send, stream, quantize)
-            else:
-                a2a.dispatch_recv(*recv, stream, out_rows)
-            return
         num_tokens = dp_x.shape[0]
         K = self._num_experts_per_token
         H = self._hidden_dim
+        if logits is not None:
+            E = self._num_local_experts * self._world_size
+            assert logits.dim() == 2 and logits.shape[0] == num_tokens and logits.shape[1] >= self._num_experts <= E
+            assert logits.stride(1) == 1 and logits.dtype in (torch.float32, torch.bfloat16)
+            if logits_bias is not None:
+                assert logits_bias.dtype == torch.float32 and logits_bias.is_contiguous()
+                assert logits_bias.numel() >= self._num_experts
 
         assert out_expert_num_tokens.shape == (self._num_local_experts,)
         assert out_expert_num_tokens.dtype == torch.int32 and out_expert_num_tokens.stride(0) == 1
         assert out_expert_x.dim() == 2 and out_expert_x.shape[1] == H
         assert out_expert_x.stride(1) == 1 and out_expert_x.dtype == self._in_dtype
-        out_rows = out_expert_x.shape[0]
-        out_x_stride = out_expert_x.stride(0) * out_expert_x.element_size()
-
         if out_expert_x_scale is not None:
             assert out_expert_x_scale.dtype == self._scale_dtype
-            out_scale = (out_expert_x_scale.data_ptr(), out_expert_x_scale.stride(1),
-                         out_expert_x_scale.stride(0))
-        else:
-            out_scale = (None, None, None)
-
         assert dp_x.shape == (num_tokens, H) and dp_x.stride(1) == 1
-        quantize = 0
-        if dp_x.dtype != self._in_dtype:
+        quantize = dp_x.dtype != self._in_dtype
+        if quantize:
             # fused quantisation: bf16 in, e4m3 + 1x128 fp32 scales on the wire
             assert dp_x.dtype == torch.bfloat16 and self._in_dtype == torch.float8_e4m3fn, (
                 f"dp_x is {dp_x.dtype}, the context was built for {self._in_dtype}")
             assert dp_x_scale is None and self._hidden_dim_scale == H // 128
             assert out_expert_x_scale is not None
-            quantize = self._quantize_mode
         if dp_x_scale is not None:
             assert self._scale_dtype is not None and self._hidden_dim_scale is not None
             assert out_expert_x_scale is not None
             assert dp_x_scale.dtype == self._scale_dtype
-            in_scale = (dp_x_scale.data_ptr(), dp_x_scale.stride(1), dp_x_scale.stride(0))
         else:
             assert quantize or (self._scale_dtype is None and self._hidden_dim_scale is None)
-            in_scale = (None, None, None)
-
         assert indices.shape == (num_tokens, K) and indices.stride(1) == 1
         assert indices.dtype == torch.uint32
         assert weights.shape == (num_tokens, K) and weights.stride(1) == 1
         assert weights.dtype == torch.float32
         if bound_m is not None:
             assert bound_m.numel() == 1 and bound_m.dtype == torch.int32
-            bound_m_ptr = bound_m.data_ptr()
-        else:
-            bound_m_ptr = None
-
-        stream = torch.cuda.current_stream().cuda_stream
-        send = (num_tokens, dp_x.data_ptr(), dp_x.stride(0) * dp_x.element_size(), *in_scale,
-                indices.data_ptr(), indices.stride(0), weights.data_ptr(), weights.stride(0),
-                bound_m_ptr)
-        recv = (out_expert_num_tokens.data_ptr(), out_expert_x.data_ptr(), out_x_stride, *out_scale)
-        if len(self._dispatch_args) > 64:
-            self._dispatch_args.clear()
-        self._dispatch_args[key] = (send, recv, out_rows, quantize)
-        if self._validate_only:
-            return
-        if do_send and do_recv:
-            a2a.dispatch(*send, *recv, stream, out_rows, quantize)
-        elif do_send:
-            a2a.dispatch_send(*send, stream, quantize)
-        else:
-            a2a.dispatch_recv(*recv, stream, out_rows)
-
-    def _dispatch_routed(self, out_expert_num_tokens, out_expert_x, out_expert_x_scale, dp_x, dp_x_scale,
-                         indices, weights, bound_m, do_send, do_recv, logits, logits_bias) -> None:
-        E = self._num_local_experts * self._world_size
-        T = dp_x.shape[0]
-        assert logits.dim() == 2 and logits.shape[0] == T and logits.shape[1] >= self._num_experts <= E
-        assert logits.stride(1) == 1 and logits.dtype in (torch.float32, torch.bfloat16)
-        if logits_bias is not None:
-            assert logits_bias.dtype == torch.float32 and logits_bias.is_contiguous()
-            assert logits_bias.numel() >= self._num_experts
-        extra = dict(logits_ptr=logits.data_ptr(), logits_stride=logits.stride(0),
-                     logits_bf16=logits.dtype == torch.bfloat16,
-                     logits_bias_ptr=None if logits_bias is None else logits_bias.data_ptr())
-        # the plain path validates everything else and caches the packed arguments
-        key = (_sig(out_expert_num_tokens), _sig(out_expert_x), _sig(out_expert_x_scale), _sig(dp_x),
-               _sig(dp_x_scale), _sig(indices), _sig(weights), _sig(bound_m))
-        if key not in self._dispatch_args:
-            self._validate_only = True
-            try:
-                self.dispatch(out_expert_num_tokens, out_expert_x, out_expert_x_scale, dp_x, dp_x_scale,
-                              indices, weights, bound_m, do_send, do_recv)
-            finally:
-                self._validate_only = False
-        send, recv, out_rows, quantize = self._dispatch_args[key]
-        stream = torch.cuda.current_stream().cuda_stream
-        a2a = self._all_to_all
-        if do_send and do_recv:
-            a2a.dispatch(*send, *recv, stream, out_rows, quantize, **extra)
-        elif do_send:
-            a2a.dispatch_send(*send, stream, quantize, **extra)
-        else:
-            a2a.dispatch_recv(*recv, stream, out_rows)
+        raise AssertionError("dispatch: unsupported arguments")
 
     # ------------------------------------------------------------------
     def combine(
@@ -455,26 +379,18 @@ class P2PAllToAll(AllToAllKernel):
         do_recv: bool = True,
         accumulate: bool = False,
     ) -> None:
-        a2a = self._all_to_all
-        assert a2a is not None
-        assert do_send or do_recv
+        assert self._all_to_all is not None
         assert not accumulate or self._dp_size == 1, "accumulate is not supported with dp_size > 1"
-        key = (_sig(out_tokens), _sig(indices), _sig(weights), _sig(expert_y), _sig(bound_m), accumulate)
-        cached = self._combine_args.get(key)
-        if cached is not None and expert_y is not None:
-            y_ptr, y_stride, num_tokens, y_dtype, y_rows, recv = cached
-            stream = torch.cuda.current_stream().cuda_stream
-            if do_send and do_recv:
-                a2a.combine(y_ptr, y_stride, num_tokens, y_dtype, *recv, stream)
-            elif do_send:
-                a2a.combine_send(y_ptr, y_stride, stream, y_dtype)
-            else:
-                a2a.combine_recv(num_tokens, y_rows, y_dtype, *recv, stream)
-            return
+        if not _torch_ops.a2a_combine(self._plan, out_tokens, indices, weights, expert_y, bound_m, do_send, do_recv,
+                                      accumulate):
+            self._reject_combine(out_tokens, indices, weights, expert_y, bound_m, do_send, do_recv)
+
+    def _reject_combine(self, out_tokens, indices, weights, expert_y, bound_m, do_send, do_recv) -> None:
+        """Raises for what the native checks of ``combine`` refused."""
+        assert do_send or do_recv
         K = self._num_experts_per_token
         H = self._hidden_dim
         num_tokens = indices.shape[0]
-
         assert out_tokens.shape == (num_tokens, H) and out_tokens.stride(1) == 1
         assert out_tokens.dtype == self._out_dtype
         assert indices.shape == (num_tokens, K) and indices.stride(1) == 1
@@ -487,31 +403,11 @@ class P2PAllToAll(AllToAllKernel):
             assert expert_y.dim() == 2 and expert_y.shape[1] == H and expert_y.stride(1) == 1
             assert expert_y.element_size() == self._out_dtype.itemsize, (
                 "expert_y must have the element size of out_dtype")
+            if expert_y.dtype not in (torch.float16, torch.bfloat16, torch.float32):
+                raise ValueError("combine supports float16, bfloat16 and float32")
         if bound_m is not None:
             assert bound_m.numel() == 1 and bound_m.dtype == torch.int32
-            bound_m_ptr = bound_m.data_ptr()
-        else:
-            bound_m_ptr = None
-
-        stream = torch.cuda.current_stream().cuda_stream
-        if expert_y is None:
-            recv = (out_tokens.data_ptr(), out_tokens.stride(0), indices.data_ptr(), indices.stride(0),
-                    weights.data_ptr(), weights.stride(0), bound_m_ptr, accumulate, stream)
-            a2a.combine_recv(num_tokens, 0, self._out_dtype, *recv)
-            return
-        y_ptr = expert_y.data_ptr()
-        y_stride = expert_y.stride(0) * expert_y.element_size()
-        recv = (out_tokens.data_ptr(), out_tokens.stride(0), indices.data_ptr(), indices.stride(0),
-                weights.data_ptr(), weights.stride(0), bound_m_ptr, accumulate)
-        if len(self._combine_args) > 64:
-            self._combine_args.clear()
-        self._combine_args[key] = (y_ptr, y_stride, num_tokens, expert_y.dtype, expert_y.shape[0], recv)
-        if do_send and do_recv:
-            a2a.combine(y_ptr, y_stride, num_tokens, expert_y.dtype, *recv, stream)
-        elif do_send:
-            a2a.combine_send(y_ptr, y_stride, stream, expert_y.dtype)
-        else:
-            a2a.combine_recv(num_tokens, expert_y.shape[0], expert_y.dtype, *recv, stream)
+        raise AssertionError("combine: unsupported arguments")
 
     # ------------------------------------------------------------------
     def barrier(self) -> None:
@@ -548,6 +444,7 @@ class P2PAllToAll(AllToAllKernel):
         # No peer may still be writing into our regions when they are unmapped.
         if self._global_group is not None:
             self._global_group.barrier()
+        self._plan = None
         self._all_to_all.destroy()      # joins the proxy thread, if any
         self._all_to_all = None
         if self._engine is not None:

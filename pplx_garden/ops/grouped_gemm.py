@@ -16,7 +16,7 @@ from typing import Optional
 
 import torch
 
-from pplx_garden import _native
+from pplx_garden import _torch_ops
 
 MODE_SWIGLU_QUANT = 0
 MODE_BF16 = 1
@@ -107,6 +107,13 @@ def grouped_fp8_gemm(
     readings for the tiles of CTA 0: epilogue tile start / first partial sums / K loop done / stored,
     MMA first issue / last commit, producer first / last load.
     """
+    fmt = _SCALE_FORMATS[scale_format]
+    if fmt == SCALES_POW2 and (wait_cycles is not None or debug_skip != 0):
+        raise ValueError("wait_cycles and debug_skip belong to the fp32-scale kernel; the pow2 kernel has trace= only")
+    if _torch_ops.grouped_fp8_gemm(a, a_scale, b, b_scale, expert_num_tokens, out, out_scale, mode, expert_padding,
+                                   error_flag, num_ctas, wait_cycles, debug_skip, trace, scatter, tile_rows, fmt):
+        return
+    # refused: say why
     assert a.dtype == torch.float8_e4m3fn and b.dtype == torch.float8_e4m3fn
     assert a.dim() == 2 and b.dim() == 3 and b.is_contiguous() and b_scale.is_contiguous()
     assert a.stride(1) == 1 and (out is None or out.stride(1) == 1)
@@ -123,15 +130,4 @@ def grouped_fp8_gemm(
         assert out is None and scatter is not None
     else:
         assert out.dtype == torch.bfloat16 and out.shape == (rows, n)
-    if _SCALE_FORMATS[scale_format] == SCALES_POW2 and (wait_cycles is not None or debug_skip != 0):
-        raise ValueError("wait_cycles and debug_skip belong to the fp32-scale kernel; the pow2 kernel has trace= only")
-    if error_flag is None:
-        error_flag = torch.zeros(1, dtype=torch.int32, device=a.device)
-    _native.grouped_fp8_gemm(
-        a.data_ptr(), a.stride(0) * a.element_size(), a_scale.data_ptr(), a_scale.stride(0), a_scale.stride(1),
-        b.data_ptr(), b_scale.data_ptr(), expert_num_tokens.data_ptr(), a.data_ptr() if out is None else out.data_ptr(),
-        16 if out is None else out.stride(0) * out.element_size(), 0 if out_scale is None else out_scale.data_ptr(),
-        0 if out_scale is None else out_scale.stride(0), error_flag.data_ptr(), e, n, k, expert_padding, rows, mode,
-        num_ctas, torch.cuda.current_stream().cuda_stream,
-        0 if wait_cycles is None else wait_cycles.data_ptr(), debug_skip,
-        0 if trace is None else trace.data_ptr(), scatter, tile_rows, _SCALE_FORMATS[scale_format])
+    raise AssertionError("grouped_fp8_gemm: unsupported arguments")
