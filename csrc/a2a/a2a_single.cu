@@ -24,6 +24,7 @@
 #include <cstdint>
 #include <type_traits>
 
+#include "../core/launch.h"
 #include "a2a_device.cuh"
 #include "a2a_ll.cuh"
 #include "a2a_kernels.h"
@@ -82,6 +83,8 @@ __global__ void __launch_bounds__(kSingleThreads, 1) dispatch_single_kernel(cons
   const A2ALocal& ws = d.ws;
   const DispatchSendArgs& a = d.send;
   const DispatchRecvArgs& r = d.recv;
+  grid_wait();
+  grid_allow_next();
   const uint32_t E = cfg.num_experts;
   const uint32_t K = cfg.topk;
   uint32_t* total = reinterpret_cast<uint32_t*>(dyn_smem + (kBulk ? kSingleWarps * 2 * kPieceBuffer : 0));
@@ -441,6 +444,8 @@ __global__ void __launch_bounds__(kBulkWarps * 32, 1) combine_bulk_kernel(const 
   const CombineRecvArgs& a = c.recv;
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   const uint32_t K = cfg.topk;
+  grid_wait();
+  grid_allow_next();
   const uint32_t T = bounded_tokens(cfg, a.num_tokens, a.bound_m);
   const uint32_t epoch = a.external ? read_epoch(c.ws, 1) : 0u;
   uint64_t* const bars = s_bars[warp];
@@ -530,6 +535,8 @@ __global__ void __launch_bounds__(kCombineThreads, 1) combine_single_kernel(cons
   const CombineRecvArgs& a = c.recv;
   const uint32_t K = cfg.topk;
   const uint32_t lane = threadIdx.x & 31u;
+  grid_wait();
+  grid_allow_next();
   const int T = bounded_tokens(cfg, a.num_tokens, a.bound_m);
   const uint32_t epoch = a.external ? read_epoch(ws, 1) : 0u;
   const bool go = combine_ready(c, T);
@@ -625,7 +632,7 @@ cudaError_t a2a_launch_dispatch_single(const A2AConfig& cfg, const A2ALocal& ws,
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
   }
-  return cudaLaunchKernel(kernel, dim3(blocks), dim3(kSingleThreads), args, smem, stream);
+  return launch_overlapped(kernel, dim3(blocks), dim3(kSingleThreads), args, smem, stream);
 }
 
 cudaError_t a2a_launch_combine_single(const A2AConfig& cfg, const A2ALocal& ws, const CombineRecvArgs& recv,
@@ -648,11 +655,11 @@ cudaError_t a2a_launch_combine_single(const A2AConfig& cfg, const A2ALocal& ws, 
       constexpr int kSmem = kBulkWarps * 2 * kBulkBuffer;
       const cudaError_t e = cudaFuncSetAttribute(combine_bulk_kernel<Y, O>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
       if (e != cudaSuccess) return e;
-      return cudaLaunchKernel(reinterpret_cast<const void*>(combine_bulk_kernel<Y, O>), dim3(cfg.num_blocks),
-                              dim3(kBulkWarps * 32), args, kSmem, stream);
+      return launch_overlapped(reinterpret_cast<const void*>(combine_bulk_kernel<Y, O>), dim3(cfg.num_blocks),
+                               dim3(kBulkWarps * 32), args, kSmem, stream);
     }
-    return cudaLaunchKernel(reinterpret_cast<const void*>(combine_single_kernel<Y, O>), dim3(cfg.num_blocks),
-                            dim3(kCombineThreads), args, 0, stream);
+    return launch_overlapped(reinterpret_cast<const void*>(combine_single_kernel<Y, O>), dim3(cfg.num_blocks),
+                             dim3(kCombineThreads), args, 0, stream);
   });
 }
 

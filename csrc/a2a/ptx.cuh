@@ -107,6 +107,12 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
   return t;
 }
 
+// Kernels launched by core/launch.h's launch_overlapped(): waits until every earlier grid of the stream
+// has ended and its writes are visible (at once where the kernel was launched in the ordinary way) ...
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// ... and lets the next such grid be brought onto the SMs as soon as there is room.
+__device__ __forceinline__ void grid_allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Named barrier over `nthreads` threads (multiple of 32). Id 0 is __syncthreads.
 __device__ __forceinline__ void bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" : : "r"(id), "r"(nthreads) : "memory");

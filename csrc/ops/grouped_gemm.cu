@@ -97,7 +97,6 @@ __device__ __forceinline__ void grouped_fp8_gemm_body(const KernelArgs& a) {
     prefetch_tensormap(&a.map_a);
     prefetch_tensormap(&a.map_b);
   }
-  if (warp == 0) build_schedule<kCtas>(a, sched, n_tiles, lane);
   if (warp == 1) {
     if constexpr (kCtas == 2) {
       tmem_alloc_pair(&tmem_base_slot, kTmemCols);
@@ -107,6 +106,9 @@ __device__ __forceinline__ void grouped_fp8_gemm_body(const KernelArgs& a) {
       tmem_relinquish();
     }
   }
+  grid_wait();   // nothing above depends on what earlier kernels wrote
+  grid_allow_next();
+  if (warp == 0) build_schedule<kCtas>(a, sched, n_tiles, lane);
   // Both CTAs' barriers and tensor memory must exist before either signals the other.
   fence_before_thread_sync();
   if constexpr (kCtas == 2) {
@@ -487,19 +489,20 @@ void PPLX_GEMM_ENTRY(const GroupedGemmParams& p, cudaStream_t stream) {
   // pair would mostly idle, and single CTAs on 128-row tiles do the same work with half the waste.
   const int tile_rows = choose_tile_rows(p);
   const int ctas = p.num_ctas > 0 ? p.num_ctas : sms;
+  void* args[] = {const_cast<KernelArgs*>(&a)};
   if (tile_rows == 256) {
     const size_t smem = static_cast<size_t>(kStages) * kStageBytesOf<2> + (kEpilogueThreads / 32) * kWarpStageBytesOf<2> + 1024;
     PPLX_CUDA_CHECK(cudaFuncSetAttribute(grouped_fp8_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(smem)));
     const int grid = std::max(2, ctas & ~1);   // whole CTA pairs
-    grouped_fp8_gemm_kernel<<<grid, kThreads, smem, stream>>>(a);
+    PPLX_CUDA_CHECK(launch_overlapped(reinterpret_cast<const void*>(grouped_fp8_gemm_kernel), dim3(grid), dim3(kThreads), args, smem, stream));
   } else {
     const size_t smem = static_cast<size_t>(kStages) * kStageBytesOf<1> + (kEpilogueThreads / 32) * kWarpStageBytesOf<1> + 1024;
     PPLX_CUDA_CHECK(cudaFuncSetAttribute(grouped_fp8_gemm_kernel_1cta, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(smem)));
-    grouped_fp8_gemm_kernel_1cta<<<std::max(1, ctas), kThreads, smem, stream>>>(a);
+    PPLX_CUDA_CHECK(launch_overlapped(reinterpret_cast<const void*>(grouped_fp8_gemm_kernel_1cta), dim3(std::max(1, ctas)), dim3(kThreads), args,
+                                      smem, stream));
   }
-  PPLX_CUDA_CHECK(cudaGetLastError());
 }
 
 }  // namespace pplx::ops

@@ -11,6 +11,7 @@
 
 #include "../core/cu_driver.h"
 #include "../core/error.h"
+#include "../core/launch.h"
 #include "grouped_gemm.h"
 #include "tcgen05.cuh"
 

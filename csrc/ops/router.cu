@@ -20,7 +20,9 @@
 #include <algorithm>
 #include <cfloat>
 
+#include "../a2a/ptx.cuh"
 #include "../core/error.h"
+#include "../core/launch.h"
 #include "router.cuh"
 
 namespace pplx::ops {
@@ -112,6 +114,8 @@ __global__ void __launch_bounds__(kMaxWarps * 32, kBlocksPerSm<PER_LANE>) topk_r
   const int E = p.num_experts, k = p.k;
   const uint32_t below = (1u << lane) - 1u;
   const bool mine = !kVec || lane * PER_LANE < E;   // a lane's run is all inside or all outside
+  grid_wait();
+  grid_allow_next();
   float bias[PER_LANE];
   #pragma unroll
   for (int j = 0; j < PER_LANE; ++j) {
@@ -217,11 +221,10 @@ void launch(const TopkRouteParams& p, int sms, cudaStream_t stream) {
   // whose warps loop, with the bias in registers.
   const int warps = p.tokens <= sms * 4 ? 1 : kMaxWarps;
   const int blocks = std::min((p.tokens + warps - 1) / warps, sms * (warps == 1 ? 4 : kBlocksPerSm<PER_LANE>));
-  if (vec) {
-    topk_route_kernel<PER_LANE, T, true><<<blocks, warps * 32, 0, stream>>>(p);
-  } else {
-    topk_route_kernel<PER_LANE, T, false><<<blocks, warps * 32, 0, stream>>>(p);
-  }
+  const void* kernel = vec ? reinterpret_cast<const void*>(topk_route_kernel<PER_LANE, T, true>)
+                           : reinterpret_cast<const void*>(topk_route_kernel<PER_LANE, T, false>);
+  void* args[] = {const_cast<TopkRouteParams*>(&p)};
+  PPLX_CUDA_CHECK(launch_overlapped(kernel, dim3(blocks), dim3(warps * 32), args, 0, stream));
 }
 
 template <typename T>
@@ -246,7 +249,6 @@ void topk_route(const TopkRouteParams& p, cudaStream_t stream) {
   PPLX_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
   if (p.logits_bf16) launch_typed<__nv_bfloat16>(p, sms, stream);
   else launch_typed<float>(p, sms, stream);
-  PPLX_CUDA_CHECK(cudaGetLastError());
 }
 
 }  // namespace pplx::ops

@@ -184,3 +184,51 @@ def test_multi_gpu_layer_matches_reference(world: int, fused: bool) -> None:
     if torch.cuda.device_count() < world:
         pytest.skip(f"needs {world} GPUs")
     assert all(ParallelLaunch(world_size=world).run(_worker, 11, fused))
+
+
+@pytest.mark.parametrize("tokens", [5, 300])
+@pytest.mark.parametrize("fused_combine", [False, True])
+def test_overlapped_launches_keep_the_order_of_a_chain(tokens: int, fused_combine: bool) -> None:
+    """Every kernel of the layer may be on the SMs before its predecessor has ended. A chain of passes,
+    each on the output of the one before, must give the same bits as with a synchronisation after every
+    step, launched one by one and replayed from a CUDA graph."""
+    from pplx_garden.models import ExpertParallelMoE, route_topk
+
+    dev = torch.device("cuda", 0)
+    H, I, E, K, steps = 512, 256, 8, 2, 12
+    layer = ExpertParallelMoE(hidden_dim=H, intermediate_dim=I, num_experts=E, num_experts_per_token=K,
+                              max_num_tokens=512, device=dev, global_group=None, init_std=0.05,
+                              fused_combine=fused_combine)
+    try:
+        gen = torch.Generator(device="cpu").manual_seed(11)
+        x0 = torch.randn((tokens, H), generator=gen).to(torch.bfloat16).to(dev)
+        gate = torch.randn((H, E), generator=gen).to(torch.bfloat16).to(dev)
+
+        def chain(sync: bool) -> torch.Tensor:
+            x = x0
+            for _ in range(steps):
+                indices, weights = route_topk(x @ gate, K)
+                if sync:
+                    torch.cuda.synchronize()
+                y = layer(x, indices, weights)
+                if sync:
+                    torch.cuda.synchronize()
+                x = torch.nn.functional.layer_norm((x + y).float(), (H,)).to(torch.bfloat16)
+            return x
+
+        want = chain(True)
+        assert torch.equal(chain(False), want)
+        stream = torch.cuda.Stream(device=dev)
+        stream.wait_stream(torch.cuda.current_stream())
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.stream(stream):
+            with torch.cuda.graph(graph, stream=stream):
+                got = chain(False)
+            for _ in range(3):
+                got.zero_()
+                graph.replay()
+                stream.synchronize()
+                assert torch.equal(got, want)
+        layer.check()
+    finally:
+        layer.destroy()
