@@ -56,7 +56,6 @@ using namespace pplx::ops::gemm_detail;
 template <int kCtas>
 __device__ __forceinline__ void grouped_fp8_gemm_body(const KernelArgs& a) {
   constexpr uint32_t kStageBytes = kStageBytesOf<kCtas>;
-  constexpr int kBBoxes = kBBoxesOf<kCtas>;
   constexpr uint32_t kWarpStageBytes = kWarpStageBytesOf<kCtas>;
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ uint64_t full_bar[kStages], empty_bar[kStages], tmem_full_bar[2], tmem_empty_bar[2];
@@ -138,29 +137,6 @@ __device__ __forceinline__ void grouped_fp8_gemm_body(const KernelArgs& a) {
         int m_pair, n_tile;
         decode_tile(sched, a.num_experts, n_tiles, t, &e, &m_pair, &n_tile);
         const int row0 = sched.row_start[e] + (kCtas * m_pair + static_cast<int>(rank)) * kBM;
-        // This CTA's half of the tile's 256 B rows (accumulator columns [128 rank, 128 rank + 128)).
-        // SwiGLU interleaves gate and up in 64-row boxes so that a thread's columns hold both.
-        // A lone CTA loads all four boxes: gate, up, gate + 64, up + 64.
-        int brow[kBBoxes];
-        if constexpr (kCtas == 2) {
-          if (swiglu) {
-            brow[0] = e * a.N + n_tile * 128 + 64 * static_cast<int>(rank);
-            brow[1] = brow[0] + I;
-          } else {
-            brow[0] = e * a.N + n_tile * kBN + 128 * static_cast<int>(rank);
-            brow[1] = brow[0] + 64;
-          }
-        } else {
-          if (swiglu) {
-            brow[0] = e * a.N + n_tile * 128;
-            brow[1] = brow[0] + I;
-            brow[2] = brow[0] + 64;
-            brow[3] = brow[1] + 64;
-          } else {
-            #pragma unroll
-            for (int i = 0; i < kBBoxes; ++i) brow[i] = e * a.N + n_tile * kBN + 64 * i;
-          }
-        }
         const int trace_row = (kProfile && a.trace != nullptr && blockIdx.x == 0 && t / num_pairs < 32) ? t / num_pairs : -1;
         if (trace_row >= 0) a.trace[trace_row * 8 + 6] = clock64();
         for (int kb = 0; kb < nkb; ++kb, ++it) {
@@ -181,19 +157,7 @@ __device__ __forceinline__ void grouped_fp8_gemm_body(const KernelArgs& a) {
           }
           if (rank == 0) mbar_expect_tx(&full_bar[s], kCtas * kStageBytes);
           const uint32_t full_s = full_leader + static_cast<uint32_t>(s) * 8u;
-          if constexpr (kCtas == 2) {
-            tma_load_2d_pair(stage, &a.map_a, kb * kBK, row0, full_s);
-          } else {
-            tma_load_2d(stage, &a.map_a, kb * kBK, row0, &full_bar[s]);
-          }
-          #pragma unroll
-          for (int i = 0; i < kBBoxes; ++i) {
-            if constexpr (kCtas == 2) {
-              tma_load_2d_pair(stage + kABytes + i * kBBoxBytes, &a.map_b, kb * kBK, brow[i], full_s);
-            } else {
-              tma_load_2d(stage + kABytes + i * kBBoxBytes, &a.map_b, kb * kBK, brow[i], &full_bar[s]);
-            }
-          }
+          load_operands<kCtas>(a, stage, kb * kBK, row0, e, n_tile, rank, full_s);
         }
         if (trace_row >= 0) a.trace[trace_row * 8 + 7] = clock64();
       }
@@ -479,7 +443,8 @@ void PPLX_GEMM_ENTRY(const GroupedGemmParams& p, cudaStream_t stream) {
   }
 #endif
   PPLX_REQUIRE(p.scale_format == kScalesFp32, "the profiled kernel takes fp32 scales only");
-  const KernelArgs a = prepare_kernel_args(p);
+  const int tile_rows = choose_tile_rows(p);
+  const KernelArgs a = prepare_kernel_args(p, tile_rows);
 
   int device = 0, sms = 0;
   PPLX_CUDA_CHECK(cudaGetDevice(&device));
@@ -487,7 +452,6 @@ void PPLX_GEMM_ENTRY(const GroupedGemmParams& p, cudaStream_t stream) {
   // Pairs of CTAs on 256-row tiles unless the experts are small: with no more than 192 rows per
   // expert on average (by capacity; the counts themselves stay on the device) the second CTA of a
   // pair would mostly idle, and single CTAs on 128-row tiles do the same work with half the waste.
-  const int tile_rows = choose_tile_rows(p);
   const int ctas = p.num_ctas > 0 ? p.num_ctas : sms;
   void* args[] = {const_cast<KernelArgs*>(&a)};
   if (tile_rows == 256) {

@@ -35,9 +35,8 @@ constexpr int kThreads = 384;
 constexpr int kFirstEpilogueWarp = 4;
 constexpr int kEpilogueThreads = 256;
 constexpr uint32_t kABytes = kBM * kBK;        // 16 KiB
-constexpr uint32_t kBBoxBytes = 64 * kBK;      // 8 KiB; a CTA of a pair holds two boxes (its half of the tile's B rows), a lone CTA four
-template <int kCtas> constexpr int kBBoxesOf = kCtas == 2 ? 2 : 4;
-template <int kCtas> constexpr uint32_t kStageBytesOf = kABytes + kBBoxesOf<kCtas> * kBBoxBytes;  // 32 / 48 KiB
+template <int kCtas> constexpr uint32_t kBBytesOf = kBN / kCtas * kBK;   // a CTA of a pair holds half of the tile's rows of B
+template <int kCtas> constexpr uint32_t kStageBytesOf = kABytes + kBBytesOf<kCtas>;  // 32 / 48 KiB
 constexpr uint32_t kBulkRowStride = 144;          // staged rows for bulk copies: 128 B + 16 B against bank conflicts
 // per epilogue warp, for coalesced output stores: 128-byte row chunks (padded for bulk copies) in
 // the pair kernel; the lone-CTA kernel's four 48 KiB stages leave room for 64-byte chunks only
@@ -102,6 +101,27 @@ __device__ __forceinline__ void decode_tile(const Schedule& s, int num_experts, 
   *e = lo;
   *m_tile = local / n_tiles;
   *n_tile = local % n_tiles;
+}
+
+// This CTA's operands of a K block, at column x: rows row0 on of A and its rows of the tile's 256 of B,
+// accumulator columns [128 rank, 128 rank + 128) for a pair and all of them for a lone CTA. map_b is
+// laid out so that these are one copy: a plain tile is a run of rows (box kBN / kCtas x 1), a SwiGLU tile
+// is 64 rows of gate and the 64 of up that belong to them (box 64 x 2 of the matrix [2 E][I][K]), so that an
+// epilogue thread's columns hold both; a lone CTA takes two such. The number of copies counts: one
+// thread issues them, a stage at a time. With boxes of 64 rows, two and four a stage, 16 experts x 1024
+// rows (fp32 scales, gate/up of 2048 x 768) took 77.8 us and take 76.5; boxes of 32 rows of A, to skip the
+// empty rows of ragged tiles, cost more than the bytes they saved (one expert of 200 rows: 37 -> 53 us).
+template <int kCtas>
+__device__ __forceinline__ void load_operands(const KernelArgs& a, uint8_t* stage, int x, int row0, int e, int n_tile,
+                                              uint32_t rank, uint32_t bar) {
+  tma_load_2d<kCtas>(stage, &a.map_a, x, row0, bar);
+  uint8_t* const b = stage + kABytes;
+  if (a.mode == kSwiGLUQuant) {
+    tma_load_3d<kCtas>(b, &a.map_b, x, n_tile * 128 + 64 * static_cast<int>(rank), 2 * e, bar);
+    if constexpr (kCtas == 1) tma_load_3d<kCtas>(b + kBBytesOf<kCtas> / 2, &a.map_b, x, n_tile * 128 + 64, 2 * e, bar);
+  } else {
+    tma_load_3d<kCtas>(b, &a.map_b, x, n_tile * kBN + 128 * static_cast<int>(rank), e, bar);
+  }
 }
 
 // One warp writes 64 bytes per row for its 32 rows (lane = row, as tensor memory hands them out)
@@ -390,16 +410,17 @@ __device__ __forceinline__ void scatter_signal(const KernelArgs& a, const uint32
   }
 }
 
-inline CUtensorMap make_map(const void* base, uint64_t rows, uint64_t cols_bytes, uint64_t row_stride_bytes,
-                     uint32_t box_rows) {
+// Of bytes [planes][rows][cols], in boxes of kBK columns.
+inline CUtensorMap make_map(const void* base, uint32_t rank, uint64_t cols, uint64_t rows, uint64_t planes, uint64_t row_stride,
+                            uint32_t box_rows, uint32_t box_planes) {
   const CuDriver& cu = CuDriver::get();
   PPLX_REQUIRE(cu.cuTensorMapEncodeTiled != nullptr, "this CUDA driver has no cuTensorMapEncodeTiled");
   CUtensorMap map;
-  const cuuint64_t dims[2] = {cols_bytes, rows};
-  const cuuint64_t strides[1] = {row_stride_bytes};
-  const cuuint32_t box[2] = {static_cast<cuuint32_t>(kBK), box_rows};
-  const cuuint32_t elem_strides[2] = {1, 1};
-  PPLX_CU_CHECK(cu.cuTensorMapEncodeTiled(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims,
+  const cuuint64_t dims[3] = {cols, rows, planes};
+  const cuuint64_t strides[2] = {row_stride, row_stride * rows};
+  const cuuint32_t box[3] = {static_cast<cuuint32_t>(kBK), box_rows, box_planes};
+  const cuuint32_t elem_strides[3] = {1, 1, 1};
+  PPLX_CU_CHECK(cu.cuTensorMapEncodeTiled(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, rank, const_cast<void*>(base), dims,
                                           strides, box, elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
                                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE));
@@ -407,7 +428,7 @@ inline CUtensorMap make_map(const void* base, uint64_t rows, uint64_t cols_bytes
 }
 
 // Argument checks common to both kernels, and the kernel's argument block.
-inline KernelArgs prepare_kernel_args(const GroupedGemmParams& p) {
+inline KernelArgs prepare_kernel_args(const GroupedGemmParams& p, int tile_rows) {
   PPLX_REQUIRE(p.K % kBK == 0 && p.K >= kBK, "K must be a multiple of 128");
   PPLX_REQUIRE(p.num_experts >= 1 && p.num_experts <= kMaxExperts, "between 1 and 128 local experts");
   PPLX_REQUIRE(p.expert_padding >= 1, "expert_padding must be positive");
@@ -435,10 +456,10 @@ inline KernelArgs prepare_kernel_args(const GroupedGemmParams& p) {
                    p.a_stride % 16 == 0 && reinterpret_cast<uintptr_t>(p.out) % 16 == 0 && p.out_stride % 16 == 0,
                "operands must be 16-byte aligned");
   KernelArgs a{};
-  a.map_a = make_map(p.a, static_cast<uint64_t>(p.max_rows), static_cast<uint64_t>(p.K),
-                     static_cast<uint64_t>(p.a_stride), kBM);
-  a.map_b = make_map(p.b, static_cast<uint64_t>(p.num_experts) * p.N, static_cast<uint64_t>(p.K),
-                     static_cast<uint64_t>(p.K), 64);
+  const uint64_t K = p.K;
+  a.map_a = make_map(p.a, 2, K, p.max_rows, 1, p.a_stride, kBM, 1);
+  a.map_b = p.mode == kSwiGLUQuant ? make_map(p.b, 3, K, p.N / 2, 2ull * p.num_experts, K, 64, 2)
+                                   : make_map(p.b, 3, K, p.N, p.num_experts, K, kBN * 128 / tile_rows, 1);
   a.a_scale = p.a_scale;
   a.a_scale_stride_row = p.a_scale_stride_row;
   a.a_scale_stride_k = p.a_scale_stride_k;

@@ -92,7 +92,6 @@ __device__ __forceinline__ void grouped_fp8_gemm_mx_body(const KernelArgs& a) {
   constexpr int kStagesMx = kMxStagesOf<kCtas>;
   constexpr int kSfSlots = kSfSlotsOf<kCtas>;
   constexpr uint32_t kStageBytes = kStageBytesOf<kCtas>;
-  constexpr int kBBoxes = kBBoxesOf<kCtas>;
   constexpr uint32_t kWarpStageBytes = kWarpStageBytesOf<kCtas>;
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ uint64_t full_bar[kStagesMx], empty_bar[kStagesMx], sf_full_bar[kSfSlots], sf_empty_bar[kSfSlots];
@@ -167,29 +166,6 @@ __device__ __forceinline__ void grouped_fp8_gemm_mx_body(const KernelArgs& a) {
           int m_pair, n_tile;
           decode_tile(sched, a.num_experts, n_tiles, t, &e, &m_pair, &n_tile);
           const int row0 = sched.row_start[e] + (kCtas * m_pair + static_cast<int>(rank)) * kBM;
-          // This CTA's rows of B: accumulator columns [128 rank, 128 rank + 128) for a pair, all 256
-          // for a lone CTA. SwiGLU interleaves gate and up in 64-row boxes so that a thread's
-          // columns hold both.
-          int brow[kBBoxes];
-          if constexpr (kCtas == 2) {
-            if (swiglu) {
-              brow[0] = e * a.N + n_tile * 128 + 64 * static_cast<int>(rank);
-              brow[1] = brow[0] + I;
-            } else {
-              brow[0] = e * a.N + n_tile * kBN + 128 * static_cast<int>(rank);
-              brow[1] = brow[0] + 64;
-            }
-          } else {
-            if (swiglu) {
-              brow[0] = e * a.N + n_tile * 128;
-              brow[1] = brow[0] + I;
-              brow[2] = brow[0] + 64;
-              brow[3] = brow[1] + 64;
-            } else {
-              #pragma unroll
-              for (int i = 0; i < kBBoxes; ++i) brow[i] = e * a.N + n_tile * kBN + 64 * i;
-            }
-          }
           for (int kb = 0; kb < nkb; ++kb, ++it) {
             const int s = it % kStagesMx;
             const uint32_t parity = ((it / kStagesMx) & 1u) ^ 1u;
@@ -201,19 +177,7 @@ __device__ __forceinline__ void grouped_fp8_gemm_mx_body(const KernelArgs& a) {
             uint8_t* stage = tiles + static_cast<size_t>(s) * kStageBytes;
             if (rank == 0) mbar_expect_tx(&full_bar[s], kCtas * kStageBytes);
             const uint32_t full_s = full_leader + static_cast<uint32_t>(s) * 8u;
-            if constexpr (kCtas == 2) {
-              tma_load_2d_pair(stage, &a.map_a, kb * kBK, row0, full_s);
-            } else {
-              tma_load_2d(stage, &a.map_a, kb * kBK, row0, &full_bar[s]);
-            }
-            #pragma unroll
-            for (int i = 0; i < kBBoxes; ++i) {
-              if constexpr (kCtas == 2) {
-                tma_load_2d_pair(stage + kABytes + i * kBBoxBytes, &a.map_b, kb * kBK, brow[i], full_s);
-              } else {
-                tma_load_2d(stage + kABytes + i * kBBoxBytes, &a.map_b, kb * kBK, brow[i], &full_bar[s]);
-              }
-            }
+            load_operands<kCtas>(a, stage, kb * kBK, row0, e, n_tile, rank, full_s);
           }
         }
       }
@@ -513,11 +477,11 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_fp8_gemm_mx_kernel_1cta(c
 
 void grouped_fp8_gemm_mx(const GroupedGemmParams& p, cudaStream_t stream) {
   PPLX_REQUIRE(p.scale_format == kScalesPow2, "grouped_fp8_gemm_mx takes power-of-two scales");
-  const KernelArgs a = prepare_kernel_args(p);
+  const int tile_rows = choose_tile_rows(p);
+  const KernelArgs a = prepare_kernel_args(p, tile_rows);
   int device = 0, sms = 0;
   PPLX_CUDA_CHECK(cudaGetDevice(&device));
   PPLX_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-  const int tile_rows = choose_tile_rows(p);
   const int ctas = p.num_ctas > 0 ? p.num_ctas : sms;
   void* args[] = {const_cast<KernelArgs*>(&a)};
   if (tile_rows == 256) {
