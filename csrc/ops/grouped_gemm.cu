@@ -93,7 +93,7 @@ __device__ __forceinline__ void grouped_fp8_gemm_body(const KernelArgs& a) {
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     s_failed = 0;
-    prefetch_tensormap(&a.map_a);
+    for (int i = 0; i < kMapsA; ++i) prefetch_tensormap(&a.map_a[i]);
     prefetch_tensormap(&a.map_b);
   }
   if (warp == 1) {
@@ -105,6 +105,9 @@ __device__ __forceinline__ void grouped_fp8_gemm_body(const KernelArgs& a) {
       tmem_relinquish();
     }
   }
+  // operand tiles need the 1024-byte alignment of the 128-byte swizzle atom
+  uint8_t* const tiles = smem + ((1024u - (smem_u32(smem) & 1023u)) & 1023u);
+  zero_stages<kCtas>(tiles, kStages, kThreads);
   grid_wait();   // nothing above depends on what earlier kernels wrote
   grid_allow_next();
   if (warp == 0) build_schedule<kCtas>(a, sched, n_tiles, lane);
@@ -118,8 +121,6 @@ __device__ __forceinline__ void grouped_fp8_gemm_body(const KernelArgs& a) {
   fence_after_thread_sync();
   const uint32_t tmem_base = tmem_base_slot;
   const int total_tiles = sched.tile_prefix[a.num_experts];
-  // operand tiles need the 1024-byte alignment of the 128-byte swizzle atom
-  uint8_t* const tiles = smem + ((1024u - (smem_u32(smem) & 1023u)) & 1023u);
 
   if (warp < kFirstEpilogueWarp) {
     // The first warpgroup only issues copies and MMAs: it keeps kLightRegs registers per thread and
@@ -132,11 +133,12 @@ __device__ __forceinline__ void grouped_fp8_gemm_body(const KernelArgs& a) {
       long long waited = 0;
       int e = 0;
       // the leader's barriers count both CTAs' bytes
+      StageRows own, peer;
       const uint32_t full_leader = kCtas == 2 ? map_to_cta(&full_bar[0], 0) : smem_u32(&full_bar[0]);
       for (int t = pair; t < total_tiles && !s_failed; t += num_pairs) {
         int m_pair, n_tile;
         decode_tile(sched, a.num_experts, n_tiles, t, &e, &m_pair, &n_tile);
-        const int row0 = sched.row_start[e] + (kCtas * m_pair + static_cast<int>(rank)) * kBM;
+        const TileLoads<kCtas> loads(sched, swiglu, e, m_pair, n_tile, rank);
         const int trace_row = (kProfile && a.trace != nullptr && blockIdx.x == 0 && t / num_pairs < 32) ? t / num_pairs : -1;
         if (trace_row >= 0) a.trace[trace_row * 8 + 6] = clock64();
         for (int kb = 0; kb < nkb; ++kb, ++it) {
@@ -155,9 +157,8 @@ __device__ __forceinline__ void grouped_fp8_gemm_body(const KernelArgs& a) {
             if (rank == 0) mbar_arrive(&full_bar[s]);
             continue;
           }
-          if (rank == 0) mbar_expect_tx(&full_bar[s], kCtas * kStageBytes);
           const uint32_t full_s = full_leader + static_cast<uint32_t>(s) * 8u;
-          load_operands<kCtas>(a, stage, kb * kBK, row0, e, n_tile, rank, full_s);
+          loads.issue(a, stage, s, kb < kStages, kb * kBK, swiglu, rank, own, peer, &full_bar[s], full_s);
         }
         if (trace_row >= 0) a.trace[trace_row * 8 + 7] = clock64();
       }

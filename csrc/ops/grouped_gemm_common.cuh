@@ -62,7 +62,7 @@ constexpr uint32_t kTraceBlocks = 30;
 constexpr uint64_t kWaitNs = 2000000000ull;  // every mbarrier wait gives up after 2 s
 
 struct KernelArgs {
-  alignas(64) CUtensorMap map_a;
+  alignas(64) CUtensorMap map_a[5];   // boxes of 16, 32, 64, 96 and 128 rows
   alignas(64) CUtensorMap map_b;
   const float* a_scale;
   int64_t a_scale_stride_row;
@@ -103,26 +103,96 @@ __device__ __forceinline__ void decode_tile(const Schedule& s, int num_experts, 
   *n_tile = local % n_tiles;
 }
 
-// This CTA's operands of a K block, at column x: rows row0 on of A and its rows of the tile's 256 of B,
-// accumulator columns [128 rank, 128 rank + 128) for a pair and all of them for a lone CTA. map_b is
-// laid out so that these are one copy: a plain tile is a run of rows (box kBN / kCtas x 1), a SwiGLU tile
-// is 64 rows of gate and the 64 of up that belong to them (box 64 x 2 of the matrix [2 E][I][K]), so that an
+// Rows of A beyond an expert's end are zeros in shared memory. Any bytes would do for the result (a row of D
+// depends on its own row of A, and these are not stored), but the kernels run at the GPU's power limit,
+// and products with the next expert's tokens draw power that products with zeros do not: an expert
+// layer of 32 x 7168 x 2048 on 97 tokens ran at 1.24 GHz and 297 us, and does at 1.50 GHz and 276 us, and
+// on 4096 tokens (a tile in eight is half empty) 1657 -> 1585 us.
+// A tile's rows are counted in units of 16 and fetched in one copy, by the map whose box has the
+// height that covers them; the rest of a stage is filled with zeros by copies of boxes that lie outside
+// of A, which read no memory, and only where the stage's last use left something else there. Boxes of
+// one height, as many as the rows need, cost more than the bytes they saved: one expert of 200 rows 37 -> 53 us.
+constexpr uint32_t kUnitRows = 16, kUnitBytes = kUnitRows * kBK;
+constexpr uint32_t kUnits = kBM / kUnitRows;
+constexpr int kMapsA = 5;   // boxes of 1, 2, 4, 6 and 8 units: index = units / 2
+
+// Units to fetch for `rows` rows: the smallest box that holds them.
+__device__ __forceinline__ uint32_t a_units(int rows) {
+  if (rows <= 0) return 0;
+  if (rows <= 16) return 1;
+  return rows > 96 ? 8u : 2u * static_cast<uint32_t>((rows + 31) / 32);
+}
+
+// Which units of every stage's A may hold something else than zeros: those below a count, four bits a
+// stage.
+struct StageRows {
+  uint32_t dirty = 0;   // see zero_stages()
+  // The stage is about to get `units` of them; returns the count of the use before.
+  __device__ __forceinline__ uint32_t replace(int stage, uint32_t units) {
+    const uint32_t before = (dirty >> (4 * stage)) & 15u;
+    dirty ^= (before ^ units) << (4 * stage);
+    return before;
+  }
+};
+
+// All threads, before the producer's first copy: the stages' rows of A start as zeros. This happens while
+// the kernel before is still running; as copies it cost a launch of one tile a CTA 3 %.
+template <int kCtas>
+__device__ __forceinline__ void zero_stages(uint8_t* tiles, int stages, int threads) {
+  for (int i = threadIdx.x; i < stages * static_cast<int>(kABytes / 16); i += threads) {
+    const int s = i / static_cast<int>(kABytes / 16), o = i % static_cast<int>(kABytes / 16);
+    *reinterpret_cast<uint4*>(tiles + static_cast<size_t>(s) * kStageBytesOf<kCtas> + 16 * o) = make_uint4(0, 0, 0, 0);
+  }
+  fence_proxy_async_smem();
+}
+
+// The copies of a tile's operands for one CTA: its rows of A and its rows of the tile's 256 of B,
+// accumulator columns [128 rank, 128 rank + 128) for a pair and all of them for a lone CTA. map_b is laid
+// out so that these are one copy: a plain tile is a run of rows (box kBN / kCtas x 1), a SwiGLU tile is 64
+// rows of gate and the 64 of up that belong to them (box 64 x 2 of the matrix [2 E][I][K]), so that an
 // epilogue thread's columns hold both; a lone CTA takes two such. The number of copies counts: one
 // thread issues them, a stage at a time. With boxes of 64 rows, two and four a stage, 16 experts x 1024
-// rows (fp32 scales, gate/up of 2048 x 768) took 77.8 us and take 76.5; boxes of 32 rows of A, to skip the
-// empty rows of ragged tiles, cost more than the bytes they saved (one expert of 200 rows: 37 -> 53 us).
+// rows (fp32 scales, gate/up of 2048 x 768) took 77.8 us and take 76.5.
 template <int kCtas>
-__device__ __forceinline__ void load_operands(const KernelArgs& a, uint8_t* stage, int x, int row0, int e, int n_tile,
-                                              uint32_t rank, uint32_t bar) {
-  tma_load_2d<kCtas>(stage, &a.map_a, x, row0, bar);
-  uint8_t* const b = stage + kABytes;
-  if (a.mode == kSwiGLUQuant) {
-    tma_load_3d<kCtas>(b, &a.map_b, x, n_tile * 128 + 64 * static_cast<int>(rank), 2 * e, bar);
-    if constexpr (kCtas == 1) tma_load_3d<kCtas>(b + kBBytesOf<kCtas> / 2, &a.map_b, x, n_tile * 128 + 64, 2 * e, bar);
-  } else {
-    tma_load_3d<kCtas>(b, &a.map_b, x, n_tile * kBN + 128 * static_cast<int>(rank), e, bar);
+struct TileLoads {
+  int row0, b_row, b_plane;
+  uint32_t units, peer_units;   // of A: this CTA's and, for a pair's leader, its peer's
+
+  __device__ __forceinline__ TileLoads(const Schedule& sched, bool swiglu, int e, int m_pair, int n_tile, uint32_t rank) {
+    const int m0 = (kCtas * m_pair + static_cast<int>(rank)) * kBM;
+    row0 = sched.row_start[e] + m0;
+    units = a_units(sched.count[e] - m0);
+    peer_units = kCtas == 2 ? a_units(sched.count[e] - m0 - kBM) : 0u;
+    b_row = swiglu ? n_tile * 128 + 64 * static_cast<int>(rank) : n_tile * kBN + 128 * static_cast<int>(rank);
+    b_plane = swiglu ? 2 * e : e;
   }
-}
+
+  // The K block at column x into stage s. `full` is the stage's mbarrier and `bar` the leader's, which
+  // counts both CTAs' bytes, as a .shared::cluster address. `first`: the stage's first use in this tile.
+  __device__ __forceinline__ void issue(const KernelArgs& a, uint8_t* stage, int s, bool first, int x, bool swiglu,
+                                        uint32_t rank, StageRows& own, StageRows& peer, uint64_t* full, uint32_t bar) const {
+    uint32_t own_before = units, peer_before = peer_units;
+    if (first) {
+      own_before = own.replace(s, units);
+      if (kCtas == 2) peer_before = peer.replace(s, peer_units);
+    }
+    if (rank == 0) {
+      mbar_expect_tx(full, (max(own_before, units) + max(peer_before, peer_units)) * kUnitBytes + kCtas * kBBytesOf<kCtas>);
+    }
+    if (units != 0) tma_load_2d<kCtas>(stage, &a.map_a[units / 2], x, row0, bar);
+    uint8_t* const b = stage + kABytes;
+    tma_load_3d<kCtas>(b, &a.map_b, x, b_row, b_plane, bar);
+    if (kCtas == 1 && swiglu) tma_load_3d<kCtas>(b + kBBytesOf<kCtas> / 2, &a.map_b, x, b_row + 64, b_plane, bar);
+    if (own_before > units) {
+      // at most two boxes: an even run of units and an odd one at its end
+      uint32_t u = units;
+      const uint32_t n = own_before - u == 1 ? 1u : (own_before - u) & ~1u;
+      tma_load_2d<kCtas>(stage + u * kUnitBytes, &a.map_a[n / 2], x, a.max_rows, bar);
+      u += n;
+      if (u < own_before) tma_load_2d<kCtas>(stage + u * kUnitBytes, &a.map_a[0], x, a.max_rows, bar);
+    }
+  }
+};
 
 // One warp writes 64 bytes per row for its 32 rows (lane = row, as tensor memory hands them out)
 // with coalesced stores: the rows are transposed through a 2 KiB staging buffer so that one store
@@ -457,7 +527,9 @@ inline KernelArgs prepare_kernel_args(const GroupedGemmParams& p, int tile_rows)
                "operands must be 16-byte aligned");
   KernelArgs a{};
   const uint64_t K = p.K;
-  a.map_a = make_map(p.a, 2, K, p.max_rows, 1, p.a_stride, kBM, 1);
+  for (int i = 0; i < kMapsA; ++i) {
+    a.map_a[i] = make_map(p.a, 2, K, p.max_rows, 1, p.a_stride, i == 0 ? kUnitRows : 2 * i * kUnitRows, 1);
+  }
   a.map_b = p.mode == kSwiGLUQuant ? make_map(p.b, 3, K, p.N / 2, 2ull * p.num_experts, K, 64, 2)
                                    : make_map(p.b, 3, K, p.N, p.num_experts, K, kBN * 128 / tile_rows, 1);
   a.a_scale = p.a_scale;

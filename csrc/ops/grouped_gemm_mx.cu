@@ -124,7 +124,7 @@ __device__ __forceinline__ void grouped_fp8_gemm_mx_body(const KernelArgs& a) {
     mbar_init(&tmem_empty_bar, kCtas * kEpilogueThreads / 32);   // the epilogue warps of every CTA of the tile (the leader's copy is used)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     s_failed = 0;
-    prefetch_tensormap(&a.map_a);
+    for (int i = 0; i < kMapsA; ++i) prefetch_tensormap(&a.map_a[i]);
     prefetch_tensormap(&a.map_b);
   }
   if (warp == 1) {
@@ -136,6 +136,9 @@ __device__ __forceinline__ void grouped_fp8_gemm_mx_body(const KernelArgs& a) {
       tmem_relinquish();
     }
   }
+  // operand tiles need the 1024-byte alignment of the 128-byte swizzle atom
+  uint8_t* const tiles = smem + ((1024u - (smem_u32(smem) & 1023u)) & 1023u);
+  zero_stages<kCtas>(tiles, kStagesMx, kThreads);
   grid_wait();   // nothing above depends on what earlier kernels wrote
   grid_allow_next();
   if (warp == 0) build_schedule<kCtas>(a, sched, n_tiles, lane);
@@ -149,7 +152,6 @@ __device__ __forceinline__ void grouped_fp8_gemm_mx_body(const KernelArgs& a) {
   fence_after_thread_sync();
   const uint32_t tmem_base = tmem_base_slot;
   const int total_tiles = sched.tile_prefix[a.num_experts];
-  uint8_t* const tiles = smem + ((1024u - (smem_u32(smem) & 1023u)) & 1023u);
   uint8_t* const warp_stages = tiles + static_cast<size_t>(kStagesMx) * kStageBytes;
   uint8_t* const sf_slots = warp_stages + (kEpilogueThreads / 32) * kWarpStageBytes;
   uint8_t* const raw_slots = sf_slots + kSfSlots * kSfSlotBytes;
@@ -161,11 +163,12 @@ __device__ __forceinline__ void grouped_fp8_gemm_mx_body(const KernelArgs& a) {
       if (lane == 0) {
         uint32_t it = 0;
         int e = 0;
+        StageRows own, peer;
         const uint32_t full_leader = kCtas == 2 ? map_to_cta(&full_bar[0], 0) : smem_u32(&full_bar[0]);
         for (int t = pair; t < total_tiles && !s_failed; t += num_pairs) {
           int m_pair, n_tile;
           decode_tile(sched, a.num_experts, n_tiles, t, &e, &m_pair, &n_tile);
-          const int row0 = sched.row_start[e] + (kCtas * m_pair + static_cast<int>(rank)) * kBM;
+          const TileLoads<kCtas> loads(sched, swiglu, e, m_pair, n_tile, rank);
           for (int kb = 0; kb < nkb; ++kb, ++it) {
             const int s = it % kStagesMx;
             const uint32_t parity = ((it / kStagesMx) & 1u) ^ 1u;
@@ -175,9 +178,8 @@ __device__ __forceinline__ void grouped_fp8_gemm_mx_body(const KernelArgs& a) {
               break;
             }
             uint8_t* stage = tiles + static_cast<size_t>(s) * kStageBytes;
-            if (rank == 0) mbar_expect_tx(&full_bar[s], kCtas * kStageBytes);
             const uint32_t full_s = full_leader + static_cast<uint32_t>(s) * 8u;
-            load_operands<kCtas>(a, stage, kb * kBK, row0, e, n_tile, rank, full_s);
+            loads.issue(a, stage, s, kb < kStagesMx, kb * kBK, swiglu, rank, own, peer, &full_bar[s], full_s);
           }
         }
       }

@@ -118,3 +118,25 @@ def test_swiglu_quant_epilogue(counts, K, I, padding, tile_rows, scales) -> None
             assert ((ratio >= 0.98) & (ratio <= 2.04)).all(), f"expert {e}: scale is not the next power of two"
         else:
             torch.testing.assert_close(out_s[start:start + n], want_scale, rtol=2e-2, atol=1e-8)
+
+
+@pytest.mark.parametrize("K", [128, 384, 1152])   # fewer K blocks than stages, and more
+@pytest.mark.parametrize("tile_rows", [128, 256])
+@pytest.mark.parametrize("scales", ["fp32", "pow2"])
+def test_tiles_of_all_heights_in_turn(K, tile_rows, scales) -> None:
+    """One CTA (or pair) takes all tiles, so that its stages hold taller and shorter ones after one
+    another: a box of A and the zeros below it at every height where another box is chosen. The rows of A
+    are small integers, so that every sum is exact and one stray row or box shows."""
+    counts = [300, 1, 129, 16, 250, 17, 0, 96, 97, 33, 64, 65, 32, 128, 145, 224, 225, 256, 15]
+    aq, a_s, bq, b_s, cnt, starts, rows = _make(counts, K, 256, 1, seed=5, unit_scales=True, pow2=True)
+    out = torch.full((rows, 256), float("nan"), dtype=torch.bfloat16, device=aq.device)
+    flag = torch.zeros(1, dtype=torch.int32, device=aq.device)
+    grouped_fp8_gemm(aq, a_s, bq, b_s, cnt, out, mode=MODE_BF16, error_flag=flag, num_ctas=tile_rows // 128,
+                     tile_rows=tile_rows, scale_format=scales)
+    torch.cuda.synchronize()
+    assert flag.item() == 0
+    a = dequantize_1x128(aq, a_s)
+    b = dequantize_128x128(bq, b_s)
+    for e, (start, n) in enumerate(zip(starts, counts)):
+        # products and sums of multiples of 2^-3 below 2^13 are exact in fp32; bf16 rounds them to 2^-8
+        torch.testing.assert_close(out[start:start + n].float(), a[start:start + n] @ b[e].T, rtol=2 ** -8, atol=0)
