@@ -105,6 +105,7 @@ class ExpertParallelMoE:
         # fused_combine: the down projection writes its rows into the peers' combine buffers itself
         self.fused_combine = fused_combine
         self.fused_bulk = fused_bulk   # fused_combine through the bulk-copy engine
+        self.send_tile_rows = 256 if world > 1 or fused_bulk else self.tile_rows
         assert not fused_combine or combine_mode == "per_route"
 
     def forward(self, x: torch.Tensor, indices: torch.Tensor, weights: torch.Tensor,
@@ -136,12 +137,14 @@ class ExpertParallelMoE:
     def down_and_send(self) -> None:
         """The down projection and the combine's send phase in one kernel: every output row is
         written over NVLink into the combine receive buffer of the GPU its token came from. Always
-        on 256-row tiles: their epilogue sends whole 128-byte lines, the single-CTA tiles' 64-byte
-        halves (EP2, 64 experts of about 256 rows: 80.8 against 109.2 us)."""
+        on 256-row tiles where that is another GPU: their epilogue sends whole 128-byte lines, the
+        single-CTA tiles' 64-byte halves (EP2, 64 experts of about 256 rows: 80.8 against 109.2 us).
+        A group of one rank writes its own memory and takes the tiles that suit its experts, as the
+        other GEMMs do (97 tokens on 32 experts of 7168 x 2048: 311 -> 286 us a layer)."""
         grouped_fp8_gemm(self.act, self.act_scale, self.w2, self.w2_scale, self.expert_num_tokens, None,
                          mode=MODE_BF16_SCATTER, error_flag=self.error_flag,
                          scatter=self.a2a.combine_send_external(self.fused_bulk),
-                         tile_rows=256, scale_format=self.scale_format)
+                         tile_rows=self.send_tile_rows, scale_format=self.scale_format)
 
     def down(self) -> None:
         """expert_y = act W_down^T in bf16: the rows combine sends home."""
