@@ -18,7 +18,7 @@
 //               counted on the leader's mbarrier, 128-byte swizzle) and keeps its 128 rows of the
 //               accumulator in its own tensor memory; the leader's commit (two-CTA mask) releases
 //               the stage and publishes the accumulator in both CTAs.
-//   lone CTA (128-row tiles)  cta_group::1, all four B boxes per stage; chosen when an expert's
+//   lone CTA (128-row tiles)  cta_group::1, all 256 rows of B per stage; chosen when an expert's
 //               capacity is 192 rows or less, where the second CTA of a pair would idle.
 //   warp 0      TMA producer into a four-stage shared-memory ring (the count must be even, see
 //               kStages) and, before the loop, the tile schedule from the experts' row counts
