@@ -287,6 +287,7 @@ __device__ __forceinline__ void grouped_fp8_gemm_mx_body(const KernelArgs& a) {
       // issue cursor
       int t_issue = pair, g_issue = 0, e = 0;
       const float* arow[4] = {a.a_scale, a.a_scale, a.a_scale, a.a_scale};
+      bool wanted[4] = {false, false, false, false};
       const float* b0 = a.b_scale;
       const float* b1 = a.b_scale;
       uint32_t sf_it = 0;
@@ -300,12 +301,14 @@ __device__ __forceinline__ void grouped_fp8_gemm_mx_body(const KernelArgs& a) {
             #pragma unroll
             for (int j = 0; j < 4; ++j) {
               const int in_tile = m_tile * kBM + 32 * j + lane;
-              // Rows past the expert's count are not stored, so any finite scale will do for them,
-              // but not one shared address: with every such lane of every CTA fetching row 0, the
-              // L2 slice holding that line ran at 70 % of its request rate (3.5x the others) and
-              // the operand tiles queued behind it (64 experts x 264 rows: 163 us against 58 us
-              // for 64 x 256). Their own row, clamped to the buffer, spreads the fetches.
-              const int row = min(sched.row_start[e] + in_tile, a.max_rows - 1);
+              // Rows past the expert's count are zeros and are not stored: any scale will do for them, and
+              // what the landing slot holds is left there. Fetched from one shared row, they made a hot
+              // line in L2 (64 experts x 264 rows: 163 us against 58 us for 64 x 256); from their own row,
+              // clamped to the buffer, still one for the last experts of a small buffer, and five times the
+              // requests of a decode tile of 24 rows. 32 experts with one row on average, 7168 x 2048
+              // gate/up: 167 us with clamped rows, 105 without any.
+              const int row = sched.row_start[e] + in_tile;
+              wanted[j] = in_tile < sched.count[e] && row < a.max_rows;
               arow[j] = a.a_scale + static_cast<int64_t>(row) * a.a_scale_stride_row;
             }
             // B's 128-row blocks behind the accumulator columns. SwiGLU: every 128 columns are 64 of
@@ -319,13 +322,15 @@ __device__ __forceinline__ void grouped_fp8_gemm_mx_body(const KernelArgs& a) {
           const int kb0 = 4 * g_issue;
           if (vec_ok && kb0 + 4 <= nkb) {
             #pragma unroll
-            for (int j = 0; j < 4; ++j) cp_async_16(raw + (32 * j + lane) * 16, arow[j] + kb0);
+            for (int j = 0; j < 4; ++j) {
+              if (wanted[j]) cp_async_16(raw + (32 * j + lane) * 16, arow[j] + kb0);
+            }
           } else {
             #pragma unroll
             for (int j = 0; j < 4; ++j) {
               #pragma unroll
               for (int k = 0; k < 4; ++k) {
-                if (kb0 + k < nkb) cp_async_4(raw + (32 * j + lane) * 16 + 4 * k, arow[j] + (kb0 + k) * a.a_scale_stride_k);
+                if (wanted[j] && kb0 + k < nkb) cp_async_4(raw + (32 * j + lane) * 16 + 4 * k, arow[j] + (kb0 + k) * a.a_scale_stride_k);
               }
             }
           }
