@@ -67,8 +67,8 @@ constexpr uint32_t kPieceBuffer = kPieceBytes + kPieceScales * sizeof(float);   
 __device__ __forceinline__ Vec16 load_quantised(const uint8_t* src, uint32_t i, uint32_t nvec, bool pow2, float* scale) {
   Vec16 lo = {0, 0, 0, 0}, hi = {0, 0, 0, 0};
   if (i < nvec) {
-    lo = ld_input_v4(src + 32ull * i);
-    hi = ld_input_v4(src + 32ull * i + 16);
+    lo = ld_after_wait_v4(src + 32ull * i);
+    hi = ld_after_wait_v4(src + 32ull * i + 16);
   }
   return quantize16(lo, hi, scale, pow2);
 }
@@ -130,8 +130,23 @@ __global__ void __launch_bounds__(kSingleThreads, 1) dispatch_single_kernel(cons
   auto load = [&](uint32_t u) {   // not kBulk
     const uint32_t i = (c0 + u % nc) * 32 + lane;
     if constexpr (kQuant) piece = load_quantised(source(u), i, nvec, pow2, &piece_scale);
-    else if (i < nvec) piece = ld_input_v4(source(u) + 16ull * i);
+    else if (i < nvec) piece = ld_after_wait_v4(source(u) + 16ull * i);
   };
+  // Nor does the routing table's count depend on anything above: its first loads are under way while the
+  // status word comes in. They have to stand here: below, the barrier would hold them back.
+  const uint32_t routes = static_cast<uint32_t>(T) * K;
+  const bool vector_indices = a.indices_stride == K && (reinterpret_cast<uintptr_t>(a.indices) & 15u) == 0;
+  const uint32_t quads = vector_indices ? routes / 4 : 0u;
+  constexpr uint32_t kQuads = 4;
+  Vec16 quad[kQuads];
+  auto load_quads = [&](uint32_t q0) {
+    #pragma unroll
+    for (uint32_t u = 0; u < kQuads; ++u) {
+      const uint32_t q = q0 + u * kSingleThreads;
+      if (q < quads) quad[u] = ld_after_wait_v4(a.indices + 4ull * q);
+    }
+  };
+  load_quads(threadIdx.x);
   const bool failed = ws.status[0] != 0;
   if constexpr (kBulk && !kQuant) {
     if (lane == 0) {
@@ -156,15 +171,18 @@ __global__ void __launch_bounds__(kSingleThreads, 1) dispatch_single_kernel(cons
     if (e < E) atomicAdd(earlier ? &next[e] : &total[e], 1u);
     else if (blockIdx.x == 0) report(ws, kStatusBadExpertIndex, kPhaseDispatchSend, t, e);
   };
-  const uint32_t routes = static_cast<uint32_t>(T) * K;
-  if (a.indices_stride == K && (reinterpret_cast<uintptr_t>(a.indices) & 15u) == 0) {
-    const uint32_t quads = routes / 4, limit = t0 * K;
-    #pragma unroll 4
-    for (uint32_t q = threadIdx.x; q < quads; q += kSingleThreads) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(a.indices) + q);
-      const uint32_t e[4] = {v.x, v.y, v.z, v.w};
+  if (vector_indices) {
+    const uint32_t limit = t0 * K;
+    for (uint32_t q0 = threadIdx.x; q0 < quads; q0 += kQuads * kSingleThreads) {
+      if (q0 != threadIdx.x) load_quads(q0);
       #pragma unroll
-      for (int c = 0; c < 4; ++c) count(e[c], 4 * q + c < limit, (4 * q + c) / K);
+      for (uint32_t u = 0; u < kQuads; ++u) {
+        const uint32_t q = q0 + u * kSingleThreads;
+        if (q >= quads) break;
+        const uint32_t e[4] = {quad[u].x, quad[u].y, quad[u].z, quad[u].w};
+        #pragma unroll
+        for (uint32_t c = 0; c < 4; ++c) count(e[c], 4 * q + c < limit, (4 * q + c) / K);
+      }
     }
     const uint32_t i = quads * 4 + threadIdx.x;
     if (i < routes) count(a.indices[i], i < limit, i / K);

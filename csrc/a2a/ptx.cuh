@@ -19,12 +19,24 @@ struct alignas(16) Vec16 {
 };
 
 // Read-only input that no kernel in flight writes (user tensors): non-coherent
-// path, do not pollute L1.
+// path, do not pollute L1. Not for kernels launched by core/launch.h's launch_overlapped(): these
+// are on the SMs while their predecessor still writes what they are going to read.
 __device__ __forceinline__ Vec16 ld_input_v4(const void* p) {
   Vec16 v;
   asm volatile("ld.global.nc.L1::no_allocate.L2::256B.v4.u32 {%0,%1,%2,%3}, [%4];"
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                : "l"(p));
+  return v;
+}
+
+// The same input read by a kernel of launch_overlapped(), after grid_wait(): coherent (weak) loads, which
+// stay behind the wait.
+__device__ __forceinline__ Vec16 ld_after_wait_v4(const void* p) {
+  Vec16 v;
+  asm volatile("ld.global.L1::no_allocate.L2::256B.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p)
+               : "memory");
   return v;
 }
 

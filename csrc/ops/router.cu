@@ -51,40 +51,34 @@ __device__ __forceinline__ void store_candidate(uint32_t key, uint32_t bound, ui
       : "memory");
 }
 
-// PER_LANE consecutive elements of a row as floats.
-template <int PER_LANE>
-__device__ __forceinline__ void load_run(const float* p, float (&v)[PER_LANE]) {
-  if constexpr (PER_LANE % 4 == 0) {
-    #pragma unroll
-    for (int j = 0; j < PER_LANE; j += 4) {
-      const float4 q = __ldg(reinterpret_cast<const float4*>(p + j));
-      v[j] = q.x; v[j + 1] = q.y; v[j + 2] = q.z; v[j + 3] = q.w;
-    }
+// N (1, 2 or 4) consecutive words, by a coherent load that stays behind grid_wait().
+template <int N>
+__device__ __forceinline__ void load_words(const void* p, uint32_t* w) {
+  if constexpr (N == 4) {
+    asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "l"(p) : "memory");
+  } else if constexpr (N == 2) {
+    asm volatile("ld.global.v2.u32 {%0,%1}, [%2];" : "=r"(w[0]), "=r"(w[1]) : "l"(p) : "memory");
   } else {
-    const float2 q = __ldg(reinterpret_cast<const float2*>(p));
-    v[0] = q.x; v[1] = q.y;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(w[0]) : "l"(p) : "memory");
   }
 }
-template <int PER_LANE>
-__device__ __forceinline__ void load_run(const __nv_bfloat16* p, float (&v)[PER_LANE]) {
-  constexpr int kWords = PER_LANE / 2;
+
+// PER_LANE consecutive elements of a row as floats.
+template <int PER_LANE, typename T>
+__device__ __forceinline__ void load_run(const T* p, float (&v)[PER_LANE]) {
+  constexpr int kWords = PER_LANE * static_cast<int>(sizeof(T)) / 4;
+  constexpr int kVec = kWords < 4 ? kWords : 4;
   uint32_t w[kWords];
-  if constexpr (kWords % 4 == 0) {
-    #pragma unroll
-    for (int j = 0; j < kWords; j += 4) {
-      const uint4 q = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint32_t*>(p) + j));
-      w[j] = q.x; w[j + 1] = q.y; w[j + 2] = q.z; w[j + 3] = q.w;
-    }
-  } else if constexpr (kWords == 2) {
-    const uint2 q = __ldg(reinterpret_cast<const uint2*>(p));
-    w[0] = q.x; w[1] = q.y;
-  } else {
-    w[0] = __ldg(reinterpret_cast<const uint32_t*>(p));
-  }
+  #pragma unroll
+  for (int j = 0; j < kWords; j += kVec) load_words<kVec>(reinterpret_cast<const uint32_t*>(p) + j, w + j);
   #pragma unroll
   for (int j = 0; j < kWords; ++j) {
-    v[2 * j] = __uint_as_float(w[j] << 16);
-    v[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
+    if constexpr (sizeof(T) == 4) {
+      v[j] = __uint_as_float(w[j]);
+    } else {
+      v[2 * j] = __uint_as_float(w[j] << 16);
+      v[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
+    }
   }
 }
 
