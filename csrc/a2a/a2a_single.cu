@@ -147,7 +147,13 @@ __global__ void __launch_bounds__(kSingleThreads, 1) dispatch_single_kernel(cons
     }
   };
   load_quads(threadIdx.x);
-  const bool failed = ws.status[0] != 0;
+  if constexpr (!kBulk) {
+    if (unit < units) load(unit);
+  }
+  // One thread reads the status word for its block: block 0 of this very launch may write it (an expert
+  // that does not exist, rows that do not fit), and a block that starts late must not be of two minds.
+  __shared__ uint32_t s_failed;
+  if (threadIdx.x == 0) s_failed = *reinterpret_cast<volatile const uint32_t*>(&ws.status[0]);
   if constexpr (kBulk && !kQuant) {
     if (lane == 0) {
       mbar_init(&s_bars[warp][0], 1);
@@ -155,17 +161,14 @@ __global__ void __launch_bounds__(kSingleThreads, 1) dispatch_single_kernel(cons
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncwarp();
-    if (!failed) fetch(unit, 0);
-  } else if constexpr (!kBulk) {
-    if (unit < units) load(unit);
-  }
-
-  if (failed) {   // an earlier failure, for all blocks alike: the word is never cleared
-    if (blockIdx.x == 0 && threadIdx.x == 0) ws.single_done[0] += 1;
-    return;
   }
   for (uint32_t i = threadIdx.x; i < 2 * E; i += kSingleThreads) total[i] = 0;
   __syncthreads();
+  if (s_failed != 0) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) ws.single_done[0] += 1;
+    return;
+  }
+  if constexpr (kBulk && !kQuant) fetch(unit, 0);
   // ---- routes per expert, those of earlier blocks' tokens apart ----
   auto count = [&](uint32_t e, bool earlier, uint32_t t) {
     if (e < E) atomicAdd(earlier ? &next[e] : &total[e], 1u);
@@ -367,27 +370,29 @@ struct SingleCombine {
   uint32_t segment;           // combine_bulk_kernel: bytes of each row that a warp reduces at a time
 };
 
-// Whether the rows may be reduced; called by all threads of every block, before anything else.
+// Whether the rows may be reduced; called by all threads of every block, before any of them is read. One
+// thread decides for its block, as in dispatch: the status word may change while the block looks at it.
 __device__ __forceinline__ bool combine_ready(const SingleCombine& c, int T) {
   const A2ALocal& ws = c.ws;
-  bool go = ws.status[0] == 0;
-  if (c.recv.external) {
-    __shared__ uint32_t s_arrived;
-    if (threadIdx.x == 0) {
+  __shared__ uint32_t s_go;
+  if (threadIdx.x == 0) {
+    bool go = *reinterpret_cast<volatile const uint32_t*>(&ws.status[0]) == 0;
+    if (c.recv.external) {
       const uint32_t expected = read_epoch(ws, 2) + 1;
       uint64_t waited;
-      s_arrived = wait_flag(c.arrived, expected, c.cfg.wait_limit_ns, &waited) ? 1u : 0u;
-      if (!s_arrived) report(ws, kStatusWaitTimeout, kPhaseCombineRecv, 0, expected);
+      const bool arrived = wait_flag(c.arrived, expected, c.cfg.wait_limit_ns, &waited);
+      if (!arrived) report(ws, kStatusWaitTimeout, kPhaseCombineRecv, 0, expected);
       if (blockIdx.x == 0) atomicMax(&ws.stats[3], static_cast<unsigned long long>(waited));
+      go = go && arrived;
+    } else if (static_cast<uint32_t>(T) > ws.expert_meta[1]) {
+      // rows of tokens that were not dispatched never come
+      if (go) report(ws, kStatusWaitTimeout, kPhaseCombineRecv, ws.expert_meta[1], T);
+      go = false;
     }
-    __syncthreads();
-    go = go && s_arrived != 0;
-  } else if (static_cast<uint32_t>(T) > ws.expert_meta[1]) {
-    // rows of tokens that were not dispatched never come
-    if (threadIdx.x == 0 && go) report(ws, kStatusWaitTimeout, kPhaseCombineRecv, ws.expert_meta[1], T);
-    go = false;
+    s_go = go ? 1u : 0u;
   }
-  return go;
+  __syncthreads();
+  return s_go != 0;
 }
 
 __device__ __forceinline__ void combine_finish(const SingleCombine& c, uint32_t epoch) {
@@ -473,27 +478,27 @@ __global__ void __launch_bounds__(kBulkWarps * 32, 1) combine_bulk_kernel(const 
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncwarp();
+  constexpr int N = VecElems<Y>::N;   // elements of a 16-byte vector
+  const uint32_t row_bytes = static_cast<uint32_t>(cfg.hidden_dim) * sizeof(Y);
+  const uint32_t seg = c.segment;     // bytes of every row in a piece, a multiple of 512
+  const uint32_t pieces = (row_bytes + seg - 1) / seg;
+  const uint32_t jobs = T * pieces;
+  const uint32_t step = gridDim.x * kBulkWarps;
+  // Routes are fetched one job before the rows, rows one job before they are reduced.
+  uint32_t job = blockIdx.x * kBulkWarps + warp;   // the warps of a block work on neighbouring pieces
+  uint32_t row, next_row;
+  float w, next_w;
+  auto route = [&](uint32_t j, uint32_t* r, float* wt) {
+    *r = kNoSlot;
+    *wt = 0.f;
+    if (j < jobs) combine_route(c, j / pieces, lane, r, wt);
+  };
+  route(job, &row, &w);
   if (combine_ready(c, T)) {
     // rows of a kernel that is still running on another stream: written by plain stores that the
     // arrival counter covers, read by the bulk-copy engine below
     if (a.external) asm volatile("fence.proxy.async;" ::: "memory");
-    constexpr int N = VecElems<Y>::N;   // elements of a 16-byte vector
-    const uint32_t row_bytes = static_cast<uint32_t>(cfg.hidden_dim) * sizeof(Y);
-    const uint32_t seg = c.segment;     // bytes of every row in a piece, a multiple of 512
-    const uint32_t pieces = (row_bytes + seg - 1) / seg;
-    const uint32_t jobs = T * pieces;
-    const uint32_t step = gridDim.x * kBulkWarps;
     uint8_t* const buffers = dyn_smem + warp * 2 * kBulkBuffer;
-
-    // Routes are fetched one job before the rows, rows one job before they are reduced.
-    uint32_t job = blockIdx.x * kBulkWarps + warp;   // the warps of a block work on neighbouring pieces
-    uint32_t row, next_row;
-    float w, next_w;
-    auto route = [&](uint32_t j, uint32_t* r, float* wt) {
-      *r = kNoSlot;
-      *wt = 0.f;
-      if (j < jobs) combine_route(c, j / pieces, lane, r, wt);
-    };
     auto fetch = [&](uint32_t j, uint32_t r, uint32_t slot) -> uint32_t {   // returns which rows come
       const uint32_t have = __ballot_sync(0xffffffffu, r != kNoSlot);
       if (have != 0) {
@@ -508,7 +513,6 @@ __global__ void __launch_bounds__(kBulkWarps * 32, 1) combine_bulk_kernel(const 
       }
       return have;
     };
-    route(job, &row, &w);
     uint32_t have = fetch(job, row, 0);
     route(job + step, &next_row, &next_w);
     uint32_t slot = 0, parities = 0;
@@ -557,18 +561,19 @@ __global__ void __launch_bounds__(kCombineThreads, 1) combine_single_kernel(cons
   grid_allow_next();
   const int T = bounded_tokens(cfg, a.num_tokens, a.bound_m);
   const uint32_t epoch = a.external ? read_epoch(ws, 1) : 0u;
-  const bool go = combine_ready(c, T);
-  if (go) {
-    const uint32_t ngran = cfg.hidden_dim / 8;
-    const uint32_t pieces = (ngran + 31) / 32;
-    constexpr int kVecs = Elem8<Y>::kBytes / 16;
-    constexpr int U = 8 / kVecs;   // rows in flight per lane
-    const uint32_t warps = gridDim.x * kCombineWarps;
-    for (uint32_t unit = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; unit < T * pieces; unit += warps) {
+  const uint32_t ngran = cfg.hidden_dim / 8;
+  const uint32_t pieces = (ngran + 31) / 32;
+  constexpr int kVecs = Elem8<Y>::kBytes / 16;
+  constexpr int U = 8 / kVecs;   // rows in flight per lane
+  const uint32_t warps = gridDim.x * kCombineWarps;
+  const uint32_t first = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  uint32_t my_row = kNoSlot;   // the first unit's routes come in while the block makes up its mind
+  float my_w = 0.f;
+  if (first < T * pieces) combine_route(c, first / pieces, lane, &my_row, &my_w);
+  if (combine_ready(c, T)) {
+    for (uint32_t unit = first; unit < T * pieces; unit += warps) {
       const uint32_t t = unit / pieces;
-      uint32_t my_row;
-      float my_w;
-      combine_route(c, t, lane, &my_row, &my_w);
+      if (unit != first) combine_route(c, t, lane, &my_row, &my_w);
       uint8_t* out_row = a.out_tokens + static_cast<uint64_t>(t) * a.out_tokens_stride * sizeof(O);
       const uint32_t g = unit % pieces * 32 + lane;
       const bool inside = g < ngran;

@@ -504,3 +504,35 @@ def test_single_rank_reports_bad_input() -> None:
             assert group.context.failed()   # the second call may already refuse
         finally:
             group.destroy()
+
+
+@pytest.mark.parametrize("tokens", [64, 1024])   # register and bulk dispatch kernels
+@pytest.mark.parametrize("quantised", [False, True])
+def test_single_rank_late_blocks_of_a_failing_launch(tokens: int, quantised: bool) -> None:
+    """Block 0 reports a bad expert while blocks of the same launch are still to start (more blocks than
+    fit the GPU): each of them takes part as a whole or not at all, and nothing lands outside the rows."""
+    hidden = 512
+    cfg = Cfg(world=1, tokens=tokens, experts=8, hidden=hidden, topk=2, in_dtype=torch.float8_e4m3fn if quantised else torch.bfloat16,
+              hidden_scale=hidden // 128 if quantised else None, out_dtype=torch.bfloat16)
+    device = torch.device("cuda", 0)
+    for _ in range(8):
+        group = _make_group(cfg, device, num_blocks=600 if tokens < 600 else 8)
+        try:
+            raw = make_rank_data(seed=1, num_experts=8, topk=2, num_tokens=tokens, hidden_dim=hidden, hidden_dim_scale=None,
+                                 in_dtype=torch.bfloat16, device=device)
+            num, _, os_, _ = _outputs(cfg, group, device)
+            rows = group.max_recv_rows
+            guarded = torch.full((rows + 64, hidden), 0x11, dtype=torch.uint8, device=device).view(torch.float8_e4m3fn) if quantised else \
+                torch.full((rows + 64, hidden), 3.0, dtype=torch.bfloat16, device=device)
+            before = guarded.view(torch.uint8).clone()
+            indices = raw.indices.view(torch.int32).clone()
+            indices[3, 1] = 8
+            group.dispatch(num, [guarded[32:32 + rows]], os_, [raw.dp_x], None, [indices.view(torch.uint32)], [raw.weights])
+            torch.cuda.synchronize()
+            assert group.context.status(0)[0] == 3
+            after = guarded.view(torch.uint8)
+            assert torch.equal(after[:32], before[:32]) and torch.equal(after[32 + rows:], before[32 + rows:])
+        except RuntimeError:
+            assert group.context.failed()   # the call itself may already see the report
+        finally:
+            group.destroy()
