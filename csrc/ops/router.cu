@@ -141,7 +141,6 @@ __global__ void __launch_bounds__(kMaxWarps * 32, kBlocksPerSm<PER_LANE>) topk_r
     uint32_t best = 0;
     #pragma unroll
     for (int j = 0; j < PER_LANE; ++j) best = max(best, key[j]);
-    ws.cand[lane] = 0;
     // at least k lanes have best >= lo, fewer than k have best >= hi; 0: fewer than k lanes hold a key
     uint32_t lo = __reduce_min_sync(0xffffffffu, best), hi = __reduce_max_sync(0xffffffffu, best);
     if (lo != 0) {
@@ -167,6 +166,9 @@ __global__ void __launch_bounds__(kMaxWarps * 32, kBlocksPerSm<PER_LANE>) topk_r
       total += __popc(lanes[j]);
     }
     if (total <= 32) {
+      // Empty places compare as none. No other lane stores to these: nothing between here and the
+      // barrier orders one lane's stores after another's.
+      if (lane >= total) ws.cand[lane] = 0;
       int before = 0;
       #pragma unroll
       for (int j = 0; j < PER_LANE; ++j) {
