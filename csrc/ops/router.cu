@@ -141,10 +141,14 @@ __global__ void __launch_bounds__(kMaxWarps * 32, kBlocksPerSm<PER_LANE>) topk_r
     uint32_t best = 0;
     #pragma unroll
     for (int j = 0; j < PER_LANE; ++j) best = max(best, key[j]);
-    // at least k lanes have best >= lo, fewer than k have best >= hi; 0: fewer than k lanes hold a key
-    uint32_t lo = __reduce_min_sync(0xffffffffu, best), hi = __reduce_max_sync(0xffffffffu, best);
-    if (lo != 0) {
-      int have = 32;
+    // At least k lanes have best >= lo, fewer than k have best >= hi. Lanes whose run of experts lies past
+    // the last one hold no key and are left out: with them in, the minimum is 0 and everything is a
+    // candidate (160 experts fill 20 lanes of 8: 32,768 tokens took 37 us, and 29 by rounds alone).
+    const int holding = __popc(__ballot_sync(0xffffffffu, best != 0));
+    uint32_t lo = __reduce_min_sync(0xffffffffu, best != 0 ? best : 0xffffffffu);
+    uint32_t hi = __reduce_max_sync(0xffffffffu, best);
+    if (holding >= k) {
+      int have = holding;
       for (int step = 0; step < 12 && have > k + 2 && hi - lo > 1; ++step) {
         const uint32_t mid = lo + (hi - lo) / 2;
         const int n = __popc(__ballot_sync(0xffffffffu, best >= mid));
@@ -155,6 +159,8 @@ __global__ void __launch_bounds__(kMaxWarps * 32, kBlocksPerSm<PER_LANE>) topk_r
           hi = mid;
         }
       }
+    } else {
+      lo = 0;   // 32 experts or fewer (see launch()): all of them are candidates
     }
     const uint32_t bound = max(lo, 1u);
     // the candidates' places in the scratch: any order will do
@@ -211,8 +217,11 @@ __global__ void __launch_bounds__(kMaxWarps * 32, kBlocksPerSm<PER_LANE>) topk_r
 template <int PER_LANE, typename T>
 void launch(const TopkRouteParams& p, int sms, cudaStream_t stream) {
   constexpr uintptr_t kAlign = std::min<size_t>(16, PER_LANE * sizeof(T));
+  // The bound needs k lanes with a key: a vector layout that fills fewer gives way to the one element a
+  // load, which fills all 32 (with 32 experts or fewer every key is a candidate and no bound is needed).
   const bool vec = p.num_experts % PER_LANE == 0 && reinterpret_cast<uintptr_t>(p.logits) % kAlign == 0 &&
-                   p.logits_stride * sizeof(T) % kAlign == 0;
+                   p.logits_stride * sizeof(T) % kAlign == 0 &&
+                   (p.num_experts / PER_LANE >= p.k || p.num_experts <= 32);
   // Few tokens: one warp a block, so that they spread over the SMs. Many: one wave of resident blocks
   // whose warps loop, with the bias in registers.
   const int warps = p.tokens <= sms * 4 ? 1 : kMaxWarps;

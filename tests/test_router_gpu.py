@@ -75,3 +75,41 @@ def test_ties_and_row_layouts(experts, k, levels, dtype):
             # __expf is good to 2 ulp + |x| ulp; differences of logits here are below 200, and what is
             # that far down has no weight
             assert torch.allclose(w.cpu(), torch.softmax(torch.gather(x, 1, want), dim=-1), rtol=1e-4, atol=1e-6)
+
+
+def _us(fn, n=30):
+    for _ in range(3):
+        fn()
+    best = float("inf")
+    for _ in range(5):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        for _ in range(n):
+            fn()
+        b.record()
+        torch.cuda.synchronize()
+        best = min(best, a.elapsed_time(b) * 1e3 / n)
+    return best
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("experts,full,k", [(96, 128, 6), (160, 256, 6), (192, 256, 8), (320, 512, 8), (384, 512, 8)])
+def test_expert_counts_that_leave_lanes_empty_cost_no_more(experts, full, k):
+    """The same number of keys a lane, fewer lanes: a token must not cost more than with all lanes filled. It
+    does, 1.4 to 1.7 times, where the bound is not found and every token takes the rounds."""
+    dev = torch.device("cuda", 0)
+    some, all_ = torch.randn((32768, experts), device=dev), torch.randn((32768, full), device=dev)
+    assert _us(lambda: topk_route(some, k)) < 1.2 * _us(lambda: topk_route(all_, k))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("experts,k", [(96, 24), (96, 25), (160, 20), (160, 21), (160, 32), (384, 24), (384, 25), (33, 32), (32, 32), (30, 20)])
+def test_k_at_the_number_of_filled_lanes(experts, k):
+    """k at and above what the vector layout fills (24, 20 and 24 lanes), where another layout takes over."""
+    dev = torch.device("cuda", 0)
+    logits = torch.randn((65, experts), generator=torch.Generator().manual_seed(experts + k)).to(dev)
+    idx, w = topk_route(logits, k)
+    want = torch.sort(logits.cpu(), dim=-1, descending=True, stable=True).indices[:, :k]
+    assert torch.equal(idx.view(torch.int32).cpu().long(), want)
+    # __expf: 2 ulp and |x| ulp, |x| below 10 here
+    assert torch.allclose(w.cpu(), torch.softmax(torch.gather(logits.cpu(), 1, want), dim=-1), rtol=1e-5, atol=1e-7)
