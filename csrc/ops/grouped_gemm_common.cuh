@@ -497,10 +497,10 @@ inline CUtensorMap make_map(const void* base, uint32_t rank, uint64_t cols, uint
   return map;
 }
 
-// Argument checks common to both kernels, and the kernel's argument block.
+// Argument checks common to both kernels (with those of choose_tile_rows(), which comes first), and the
+// kernel's argument block.
 inline KernelArgs prepare_kernel_args(const GroupedGemmParams& p, int tile_rows) {
   PPLX_REQUIRE(p.K % kBK == 0 && p.K >= kBK, "K must be a multiple of 128");
-  PPLX_REQUIRE(p.num_experts >= 1 && p.num_experts <= kMaxExperts, "between 1 and 128 local experts");
   PPLX_REQUIRE(p.expert_padding >= 1, "expert_padding must be positive");
   if (p.mode == kSwiGLUQuant) {
     PPLX_REQUIRE(p.N % 256 == 0, "SwiGLU needs N = 2 * intermediate with intermediate a multiple of 128");
@@ -559,6 +559,7 @@ inline KernelArgs prepare_kernel_args(const GroupedGemmParams& p, int tile_rows)
 // expert on average (by capacity; the counts themselves stay on the device) the second CTA of a
 // pair would mostly idle, and single CTAs on 128-row tiles do the same work with half the waste.
 inline int choose_tile_rows(const GroupedGemmParams& p) {
+  PPLX_REQUIRE(p.num_experts >= 1 && p.num_experts <= kMaxExperts, "between 1 and 128 local experts");   // divided by below
   const bool wants_pairs = p.mode == kBf16Scatter && p.scatter.bulk;   // the bulk-copy sender stages 128-byte rows
   const int tile_rows =
       p.tile_rows != 0 ? p.tile_rows : ((wants_pairs || p.max_rows / p.num_experts > 192) ? 256 : 128);

@@ -140,3 +140,16 @@ def test_tiles_of_all_heights_in_turn(K, tile_rows, scales) -> None:
     for e, (start, n) in enumerate(zip(starts, counts)):
         # products and sums of multiples of 2^-3 below 2^13 are exact in fp32; bf16 rounds them to 2^-8
         torch.testing.assert_close(out[start:start + n].float(), a[start:start + n] @ b[e].T, rtol=2 ** -8, atol=0)
+
+
+@pytest.mark.parametrize("scales", ["fp32", "pow2"])
+@pytest.mark.parametrize("experts", [0, 129])
+def test_number_of_experts_is_checked(scales, experts) -> None:
+    """Refused on the host before anything is derived from the count (the automatic tile height divides
+    by it)."""
+    dev = torch.device("cuda", 0)
+    fp8 = lambda *shape: torch.zeros(shape, dtype=torch.uint8, device=dev).view(torch.float8_e4m3fn)  # noqa: E731
+    with pytest.raises(ValueError, match="between 1 and 128 local experts"):
+        grouped_fp8_gemm(fp8(8, 128), torch.ones((8, 1), device=dev), fp8(experts, 256, 128),
+                         torch.ones((experts, 2, 1), device=dev), torch.zeros(experts, dtype=torch.int32, device=dev),
+                         torch.zeros((8, 256), dtype=torch.bfloat16, device=dev), mode=MODE_BF16, scale_format=scales)
