@@ -105,7 +105,7 @@ class ExpertParallelMoE:
         # fused_combine: the down projection writes its rows into the peers' combine buffers itself
         self.fused_combine = fused_combine
         self.fused_bulk = fused_bulk   # fused_combine through the bulk-copy engine
-        self.send_tile_rows = 256 if world > 1 or fused_bulk else self.tile_rows
+        self.world = world
         assert not fused_combine or combine_mode == "per_route"
 
     def forward(self, x: torch.Tensor, indices: torch.Tensor, weights: torch.Tensor,
@@ -141,10 +141,12 @@ class ExpertParallelMoE:
         single-CTA tiles' 64-byte halves (EP2, 64 experts of about 256 rows: 80.8 against 109.2 us).
         A group of one rank writes its own memory and takes the tiles that suit its experts, as the
         other GEMMs do (97 tokens on 32 experts of 7168 x 2048: 311 -> 286 us a layer)."""
+        # the bulk-copy sender stages 128-byte rows, which is what 256-row tiles have
+        tile_rows = 256 if self.world > 1 or self.fused_bulk else self.tile_rows
         grouped_fp8_gemm(self.act, self.act_scale, self.w2, self.w2_scale, self.expert_num_tokens, None,
                          mode=MODE_BF16_SCATTER, error_flag=self.error_flag,
                          scatter=self.a2a.combine_send_external(self.fused_bulk),
-                         tile_rows=self.send_tile_rows, scale_format=self.scale_format)
+                         tile_rows=tile_rows, scale_format=self.scale_format)
 
     def down(self) -> None:
         """expert_y = act W_down^T in bf16: the rows combine sends home."""

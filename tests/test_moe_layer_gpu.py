@@ -232,3 +232,27 @@ def test_overlapped_launches_keep_the_order_of_a_chain(tokens: int, fused_combin
         layer.check()
     finally:
         layer.destroy()
+
+
+def test_bulk_sender_switched_on_after_construction() -> None:
+    """fused_bulk is read at every call: the tiles must suit the sender that the call uses (and small
+    experts, whose other GEMMs run on 128-row tiles, must not keep it from 256-row ones)."""
+    from pplx_garden.models import ExpertParallelMoE, route_topk
+
+    dev = torch.device("cuda", 0)
+    H, I, E, K, T = 512, 256, 8, 2, 64
+    gen = torch.Generator(device="cpu").manual_seed(7)
+    x = torch.randn((T, H), generator=gen).to(torch.bfloat16).to(dev)
+    indices, weights = route_topk(torch.randn((T, E), generator=gen).to(dev), K)
+    layer = ExpertParallelMoE(hidden_dim=H, intermediate_dim=I, num_experts=E, num_experts_per_token=K,
+                              max_num_tokens=T, device=dev, global_group=None, init_std=0.05, fused_combine=True)
+    try:
+        outs = []
+        for bulk in (False, True, False):
+            layer.fused_bulk = bulk
+            outs.append(layer(x, indices, weights).clone())
+        torch.cuda.synchronize()
+        layer.check()
+        assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    finally:
+        layer.destroy()
