@@ -75,16 +75,12 @@ ImmIncResult ImmCountMap::inc(uint32_t imm, uint32_t n) {
 
 uint32_t ImmCountMap::inc_each(uint32_t imm, uint32_t n, bool* reached) {
   *reached = false;
-  {
-    std::shared_lock lock(mu_);
-    auto it = map_.find(imm);
-    if (it == map_.end()) return n;
-    Entry& e = it->second;
-    if (e.kind == Entry::Kind::kFree) {
-      e.counter->fetch_add(n, std::memory_order_acq_rel);
-      return 0;
-    }
-    if (e.kind == Entry::Kind::kExpected) {
+  std::shared_lock lock(mu_);   // for the whole batch: the counter it meets is the one that takes it
+  auto it = map_.find(imm);
+  if (it == map_.end()) return n;
+  Entry& e = it->second;
+  switch (e.kind) {
+    case Entry::Kind::kExpected: {
       int64_t have = e.counter->load(std::memory_order_acquire);
       int64_t take = 0;
       do {
@@ -93,9 +89,20 @@ uint32_t ImmCountMap::inc_each(uint32_t imm, uint32_t n, bool* reached) {
       *reached = take > 0 && have + take == e.expected;
       return n - static_cast<uint32_t>(take);
     }
+    case Entry::Kind::kFree:
+      e.counter->fetch_add(n, std::memory_order_acq_rel);
+      return 0;
+    case Entry::Kind::kFlag: {
+      // raised by the arrival that brings the counter to zero, wherever in the batch that is
+      const int64_t before = e.counter->fetch_add(n, std::memory_order_acq_rel);
+      if (before < 0 && before + n >= 0 && e.flag != nullptr) {
+        *e.flag = 1u;
+        std::atomic_thread_fence(std::memory_order_seq_cst);
+      }
+      return 0;
+    }
   }
-  for (uint32_t i = 0; i < n; ++i) inc(imm, 1);   // Flag: may pass zero on the way
-  return 0;
+  return n;
 }
 
 size_t ImmCountMap::size() const {

@@ -144,6 +144,40 @@ void test_imm_count_batches() {
   ImmCountMap none;
   bool got = true;
   CHECK(none.inc_each(5, 4, &got) == 4 && !got);
+  // a flag is raised when a batch brings its counter to zero or past it, and only then
+  for (int64_t debt : {-1, -3, -4, -5, 0, 2}) {
+    ImmCountMap map;
+    volatile uint32_t flag = 0;
+    auto cell = map.set_flag(6, &flag);
+    cell->store(debt);
+    CHECK(map.inc_each(6, 4, &got) == 0 && !got);
+    CHECK(cell->load() == debt + 4 && flag == (debt < 0 && debt + 4 >= 0 ? 1u : 0u));
+  }
+}
+
+// No arrival of a batch may be lost while its counter is installed and removed: each is either in
+// the counter or reported as having met none.
+void test_imm_count_batches_while_counters_change() {
+  ImmCountMap map;
+  constexpr uint32_t kBatches = 20000, kBatch = 64;
+  std::atomic<bool> done{false};
+  uint64_t vacant = 0, counted = 0;
+  std::thread arrivals([&] {
+    for (uint32_t i = 0; i < kBatches; ++i) {
+      bool reached = false;
+      vacant += map.inc_each(3, kBatch, &reached);
+    }
+    done = true;
+  });
+  volatile uint32_t flag = 0;
+  while (!done) {
+    auto cell = map.set_flag(3, &flag);
+    std::this_thread::yield();
+    CHECK(map.remove(3).has_value());
+    counted += static_cast<uint64_t>(cell->load());   // nobody finds the cell any more
+  }
+  arrivals.join();
+  CHECK(vacant + counted == static_cast<uint64_t>(kBatches) * kBatch);
 }
 
 void test_cpu_leases() {
@@ -630,6 +664,7 @@ int main() {
   test_defer_and_pools();
   test_imm_counts();
   test_imm_count_batches();
+  test_imm_count_batches_while_counters_change();
   test_cpu_leases();
   test_sharding();
   test_host_buffers();
