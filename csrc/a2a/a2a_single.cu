@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(kSingleThreads, 1) dispatch_single_kernel(cons
           }
         }
         bulk_commit();
-        if (kQuant && !d.bulk_scales) {
+        if (kQuant && !d.bulk_scales && os != nullptr) {
           for (uint32_t i = lane; i < bytes / 128 * K; i += 32) {
             const uint32_t row = rows[i % K], j = i / K;
             if (row != kNoSlot) {
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(kSingleThreads, 1) dispatch_single_kernel(cons
           const uint32_t row = rows[k];
           if (row == kNoSlot || i >= nvec) continue;
           st_stream_v4(r.out_x + static_cast<uint64_t>(row) * r.out_x_stride + 16ull * i, piece);
-          if (kQuant && (i & 7u) == 0) {
+          if (kQuant && os != nullptr && (i & 7u) == 0) {
             os[static_cast<int64_t>(row) * r.out_x_scale_stride_token +
                static_cast<int64_t>(i >> 3) * r.out_x_scale_stride_elem] = piece_scale;
           }
@@ -642,7 +642,8 @@ cudaError_t a2a_launch_dispatch_single(const A2AConfig& cfg, const A2ALocal& ws,
   if (!bulk && send.num_tokens > 0) {
     d.parts = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(blocks / send.num_tokens, (nvec + 31) / 32)));
   }
-  d.bulk_scales = recv.out_x_scale_stride_elem == 1 && recv.out_x_scale_stride_token % 4 == 0 &&
+  // (scales nobody asks for are not written, quantised or not)
+  d.bulk_scales = recv.out_x_scale != nullptr && recv.out_x_scale_stride_elem == 1 && recv.out_x_scale_stride_token % 4 == 0 &&
                   cfg.hidden_dim_scale % 4 == 0 && reinterpret_cast<uintptr_t>(recv.out_x_scale) % 16 == 0;
   const size_t smem = 2 * sizeof(uint32_t) * cfg.num_experts + (bulk ? kSingleWarps * 2 * kPieceBuffer : 0);
   void* args[] = {&d};

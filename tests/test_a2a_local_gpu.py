@@ -536,3 +536,29 @@ def test_single_rank_late_blocks_of_a_failing_launch(tokens: int, quantised: boo
             assert group.context.failed()   # the call itself may already see the report
         finally:
             group.destroy()
+
+
+@pytest.mark.parametrize("num_blocks", [4, 148])   # bulk and register dispatch kernels
+@pytest.mark.parametrize("split", [False, True])
+def test_single_rank_quantises_without_a_scale_output(num_blocks: int, split: bool) -> None:
+    """A caller may leave the scales of a quantising dispatch out: the rows come all the same."""
+    tokens, hidden = 600, 512   # token t goes to expert t alone, so that its row is row t
+    cfg = Cfg(world=1, tokens=tokens, experts=tokens, hidden=hidden, hidden_scale=hidden // 128, topk=1,
+              in_dtype=torch.float8_e4m3fn, out_dtype=torch.bfloat16)
+    device = torch.device("cuda", 0)
+    group = _make_group(cfg, device, num_blocks=num_blocks)
+    try:
+        x = torch.randn((tokens, hidden), generator=torch.Generator().manual_seed(1)).to(torch.bfloat16)
+        indices = torch.arange(tokens, dtype=torch.int32, device=device).view(-1, 1).view(torch.uint32)
+        weights = torch.ones((tokens, 1), device=device)
+        num, ox, _, _ = _outputs(cfg, group, device)
+        for send, recv in ([(True, False), (False, True)] if split else [(True, True)]):
+            group.dispatch(num, ox, None, [x.to(device)], None, [indices], [weights], None, send, recv)
+        torch.cuda.synchronize()
+        group.check()
+        want = oracle.quantize_1x128(x.float())[0].float()
+        # e4m3: an element at the middle of two values may round either way
+        torch.testing.assert_close(ox[0][:tokens].float().cpu(), want, rtol=0.13, atol=2 ** -9)
+        assert (num[0] == 1).all()
+    finally:
+        group.destroy()
