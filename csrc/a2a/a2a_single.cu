@@ -372,7 +372,7 @@ struct SingleCombine {
 
 // Whether the rows may be reduced; called by all threads of every block, before any of them is read. One
 // thread decides for its block, as in dispatch: the status word may change while the block looks at it.
-__device__ __forceinline__ bool combine_ready(const SingleCombine& c, int T) {
+__device__ __forceinline__ bool combine_ready(const SingleCombine& c) {
   const A2ALocal& ws = c.ws;
   __shared__ uint32_t s_go;
   if (threadIdx.x == 0) {
@@ -384,10 +384,6 @@ __device__ __forceinline__ bool combine_ready(const SingleCombine& c, int T) {
       if (!arrived) report(ws, kStatusWaitTimeout, kPhaseCombineRecv, 0, expected);
       if (blockIdx.x == 0) atomicMax(&ws.stats[3], static_cast<unsigned long long>(waited));
       go = go && arrived;
-    } else if (static_cast<uint32_t>(T) > ws.expert_meta[1]) {
-      // rows of tokens that were not dispatched never come
-      if (go) report(ws, kStatusWaitTimeout, kPhaseCombineRecv, ws.expert_meta[1], T);
-      go = false;
     }
     s_go = go ? 1u : 0u;
   }
@@ -403,21 +399,31 @@ __device__ __forceinline__ void combine_finish(const SingleCombine& c, uint32_t 
   }
 }
 
-// Lane k: where token t's k-th row is (kNoSlot: nowhere) and its weight.
-__device__ __forceinline__ void combine_route(const SingleCombine& c, uint32_t t, uint32_t lane, uint32_t* row, float* w) {
+// Lane k: where token t's k-th row is (kNoSlot: nowhere) and its weight. All 32 lanes call. The routes of
+// the combine decide what is reduced, as in the general kernels: one with an expert that does not exist
+// is left out (in the pre-reduced mode only a token with no other counts for nothing), so that a
+// caller may dispatch by bound_m and combine the padding too, or mask single routes. `dispatched`: tokens
+// that were; the rows of a later one never come.
+__device__ __forceinline__ void combine_route(const SingleCombine& c, uint32_t t, uint32_t lane, uint32_t dispatched,
+                                              uint32_t* row, float* w) {
   const A2AConfig& cfg = c.cfg;
   const CombineRecvArgs& a = c.recv;
   const uint32_t K = cfg.topk;
+  const bool per_route = cfg.combine_mode == kCombinePerRoute;
   *row = kNoSlot;
   *w = 0.f;
+  bool valid = false;
   if (lane < K) {
     const uint64_t tk = static_cast<uint64_t>(t) * K + lane;
-    if (a.external) {
-      if (a.indices[t * a.indices_stride + lane] < static_cast<uint32_t>(cfg.num_experts)) *row = static_cast<uint32_t>(tk);
-    } else {
-      *row = c.ws.route_row[tk];
-    }
-    *w = a.external || cfg.combine_mode == kCombinePerRoute ? a.weights[t * a.weights_stride + lane] : c.ws.rec_weights[tk];
+    valid = a.indices[t * a.indices_stride + lane] < static_cast<uint32_t>(cfg.num_experts);
+    if (a.external) *row = static_cast<uint32_t>(tk);
+    else if (t < dispatched) *row = c.ws.route_row[tk];
+    *w = a.external || per_route ? a.weights[t * a.weights_stride + lane] : c.ws.rec_weights[tk];
+  }
+  const uint32_t any = __ballot_sync(0xffffffffu, valid);
+  if (per_route ? !valid : any == 0) *row = kNoSlot;
+  if (!a.external && t >= dispatched && any != 0 && lane == 0) {
+    report(c.ws, kStatusWaitTimeout, kPhaseCombineRecv, t, dispatched);
   }
 }
 
@@ -471,6 +477,7 @@ __global__ void __launch_bounds__(kBulkWarps * 32, 1) combine_bulk_kernel(const 
   grid_allow_next();
   const uint32_t T = bounded_tokens(cfg, a.num_tokens, a.bound_m);
   const uint32_t epoch = a.external ? read_epoch(c.ws, 1) : 0u;
+  const uint32_t dispatched = c.ws.expert_meta[1];
   uint64_t* const bars = s_bars[warp];
   if (lane == 0) {
     mbar_init(&bars[0], 1);
@@ -491,10 +498,10 @@ __global__ void __launch_bounds__(kBulkWarps * 32, 1) combine_bulk_kernel(const 
   auto route = [&](uint32_t j, uint32_t* r, float* wt) {
     *r = kNoSlot;
     *wt = 0.f;
-    if (j < jobs) combine_route(c, j / pieces, lane, r, wt);
+    if (j < jobs) combine_route(c, j / pieces, lane, dispatched, r, wt);
   };
   route(job, &row, &w);
-  if (combine_ready(c, T)) {
+  if (combine_ready(c)) {
     // rows of a kernel that is still running on another stream: written by plain stores that the
     // arrival counter covers, read by the bulk-copy engine below
     if (a.external) asm volatile("fence.proxy.async;" ::: "memory");
@@ -561,6 +568,7 @@ __global__ void __launch_bounds__(kCombineThreads, 1) combine_single_kernel(cons
   grid_allow_next();
   const int T = bounded_tokens(cfg, a.num_tokens, a.bound_m);
   const uint32_t epoch = a.external ? read_epoch(ws, 1) : 0u;
+  const uint32_t dispatched = ws.expert_meta[1];
   const uint32_t ngran = cfg.hidden_dim / 8;
   const uint32_t pieces = (ngran + 31) / 32;
   constexpr int kVecs = Elem8<Y>::kBytes / 16;
@@ -569,11 +577,11 @@ __global__ void __launch_bounds__(kCombineThreads, 1) combine_single_kernel(cons
   const uint32_t first = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
   uint32_t my_row = kNoSlot;   // the first unit's routes come in while the block makes up its mind
   float my_w = 0.f;
-  if (first < T * pieces) combine_route(c, first / pieces, lane, &my_row, &my_w);
-  if (combine_ready(c, T)) {
+  if (first < T * pieces) combine_route(c, first / pieces, lane, dispatched, &my_row, &my_w);
+  if (combine_ready(c)) {
     for (uint32_t unit = first; unit < T * pieces; unit += warps) {
       const uint32_t t = unit / pieces;
-      if (unit != first) combine_route(c, t, lane, &my_row, &my_w);
+      if (unit != first) combine_route(c, t, lane, dispatched, &my_row, &my_w);
       uint8_t* out_row = a.out_tokens + static_cast<uint64_t>(t) * a.out_tokens_stride * sizeof(O);
       const uint32_t g = unit % pieces * 32 + lane;
       const bool inside = g < ngran;

@@ -562,3 +562,62 @@ def test_single_rank_quantises_without_a_scale_output(num_blocks: int, split: bo
         assert (num[0] == 1).all()
     finally:
         group.destroy()
+
+
+@pytest.mark.parametrize("num_blocks", [2, 148])   # bulk and register combine kernels
+@pytest.mark.parametrize("combine_mode", ["per_route", "pre_reduce"])
+def test_single_rank_combines_what_the_routes_of_the_combine_say(num_blocks: int, combine_mode: str) -> None:
+    """Routes masked between dispatch and combine, and padding past the dispatch's bound_m that the combine
+    is not told of: as the split phases, which are the general kernels, do it."""
+    tokens, hidden, topk, bound = 100, 1040, 4, 61
+    cfg = Cfg(world=1, tokens=tokens, experts=16, hidden=hidden, topk=topk, in_dtype=torch.bfloat16, out_dtype=torch.bfloat16,
+              combine_mode=combine_mode, wire="ll")   # only its combine_recv copes with rows that nobody waits for
+    device = torch.device("cuda", 0)
+    group = _make_group(cfg, device, num_blocks=num_blocks)
+    try:
+        d = _inputs(cfg, device)[0]
+        full = d.indices.view(torch.int32)
+        masked = full.clone()
+        masked[::3, 1] = -1      # single routes
+        masked[5:9] = -1         # whole tokens
+        padded = full.clone()
+        padded[bound:] = -1
+        bm = [torch.tensor([bound], dtype=torch.int32, device=device)]
+        for sent, combined, limit in ((full, masked, None), (padded, padded, bm)):
+            outs = []
+            for split in (False, True):
+                num, ox, _, out = _outputs(cfg, group, device)
+                out[0].fill_(7.0)
+                idx = [sent.view(torch.uint32)]
+                group.dispatch(num, ox, None, [d.dp_x], None, idx, [d.weights], limit)
+                ys = [act(ox[0], None).to(cfg.out_dtype)]
+                idx = [combined.view(torch.uint32)]
+                for send, recv in ([(True, False), (False, True)] if split else [(True, True)]):
+                    group.combine(out, idx, [d.weights], ys, None, send, recv)
+                torch.cuda.synchronize()
+                group.check()
+                outs.append(out[0].clone())
+            assert torch.equal(outs[0], outs[1])
+            assert torch.count_nonzero(outs[0][(combined < 0).all(dim=1)]) == 0
+    finally:
+        group.destroy()
+
+
+def test_single_rank_reports_tokens_that_were_not_dispatched() -> None:
+    cfg = Cfg(world=1, tokens=16, experts=8, hidden=64, topk=2)
+    device = torch.device("cuda", 0)
+    group = _make_group(cfg, device)
+    try:
+        d = _inputs(cfg, device)[0]
+        num, ox, _, out = _outputs(cfg, group, device)
+        group.dispatch(num, ox, None, [d.dp_x], None, [d.indices], [d.weights],
+                       [torch.tensor([9], dtype=torch.int32, device=device)])
+        try:
+            group.combine(out, [d.indices], [d.weights], [torch.zeros_like(ox[0])])
+        except (RuntimeError, TimeoutError):
+            pass   # the call itself may already see the report
+        torch.cuda.synchronize()
+        code, phase, who, _, message = group.context.status(0)
+        assert code == 1 and phase == 3 and 9 <= who < 16, message
+    finally:
+        group.destroy()
