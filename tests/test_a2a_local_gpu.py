@@ -621,3 +621,41 @@ def test_single_rank_reports_tokens_that_were_not_dispatched() -> None:
         assert code == 1 and phase == 3 and 9 <= who < 16, message
     finally:
         group.destroy()
+
+
+@pytest.mark.parametrize("num_blocks", [4, 148])   # bulk and register dispatch kernels
+@pytest.mark.parametrize("hidden,strided", [
+    (512, False), (640, False), (2048, True), (2560, False), (2688, False), (2688, True)])
+@pytest.mark.parametrize("pow2", [False, True])
+def test_single_rank_quantises_like_the_reference(num_blocks: int, hidden: int, strided: bool, pow2: bool) -> None:
+    """Fused quantisation of one rank, with one and two pieces a token, whole and ragged, the scales written
+    in bulk (a multiple of four of them) or one by one (any other number, or columns apart)."""
+    tokens, experts = 701, 701   # token t goes to experts t and t + 1: two rows an expert
+    cfg = Cfg(world=1, tokens=tokens, experts=experts, hidden=hidden, hidden_scale=hidden // 128, topk=2,
+              in_dtype=torch.float8_e4m3fn, out_dtype=torch.bfloat16)
+    device = torch.device("cuda", 0)
+    group = _make_group(cfg, device, num_blocks=num_blocks, pow2_scales=pow2)
+    try:
+        gen = torch.Generator().manual_seed(hidden)
+        x = (torch.randn((tokens, hidden), generator=gen) * torch.exp2(torch.randint(-6, 7, (tokens, 1), generator=gen))).to(torch.bfloat16)
+        x[5] = 0   # the smallest scale
+        t = torch.arange(tokens, dtype=torch.int32, device=device)
+        indices = torch.stack([t, (t + 1) % experts], dim=1).view(torch.uint32)
+        weights = torch.full((tokens, 2), 0.5, device=device)
+        num, ox, os_, _ = _outputs(cfg, group, device)
+        if strided:
+            os_ = [torch.zeros((hidden // 128, group.max_recv_rows), device=device).t()]
+        group.dispatch(num, ox, os_, [x.to(device)], None, [indices], [weights])
+        torch.cuda.synchronize()
+        group.check()
+        assert (num[0] == 2).all()
+        q, scale = oracle.quantize_1x128(x.float(), pow2=pow2)
+        # same float32 operations in the same order: bit for bit, in either order of an expert's two rows
+        want = torch.cat([q.view(torch.uint8), scale.contiguous().view(torch.uint8)], dim=1)
+        got = torch.cat([ox[0][:2 * tokens].cpu().view(torch.uint8), os_[0][:2 * tokens].cpu().contiguous().view(torch.uint8)], dim=1)
+        got = got.view(tokens, 2, -1)
+        before = want.roll(1, dims=0)
+        ok = ((got[:, 0] == want) & (got[:, 1] == before)).all(dim=1) | ((got[:, 1] == want) & (got[:, 0] == before)).all(dim=1)
+        assert ok.all(), f"experts {(~ok).nonzero().flatten().tolist()[:8]}"
+    finally:
+        group.destroy()

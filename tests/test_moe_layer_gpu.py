@@ -256,3 +256,86 @@ def test_bulk_sender_switched_on_after_construction() -> None:
         assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
     finally:
         layer.destroy()
+
+
+def test_bulk_combine_of_rows_another_kernel_sent(monkeypatch) -> None:
+    """Prefill sizes: the combine fetches the rows that the down projection sent through the bulk-copy
+    engine. Bit for bit the tokens of GEMM -> expert_y -> combine."""
+    from pplx_garden.models import ExpertParallelMoE, route_topk
+
+    monkeypatch.setenv("PPLX_A2A_BLOCKS", "4")   # the bulk kernel from 48 pieces a block: 192 tokens of one piece
+    dev = torch.device("cuda", 0)
+    H, I, E, K, T = 512, 256, 8, 3, 301
+    gen = torch.Generator(device="cpu").manual_seed(13)
+    w13, w2 = torch.randn((E, 2 * I, H), generator=gen) * 0.05, torch.randn((E, H, I), generator=gen) * 0.05
+    outs = []
+    for fused, bulk in ((False, False), (True, False), (True, True)):
+        layer = ExpertParallelMoE(hidden_dim=H, intermediate_dim=I, num_experts=E, num_experts_per_token=K,
+                                  max_num_tokens=T, device=dev, global_group=None, w13=w13, w2=w2,
+                                  fused_combine=fused, fused_bulk=bulk)
+        try:
+            passes = []
+            for step in range(3):
+                g2 = torch.Generator(device="cpu").manual_seed(step)
+                x = torch.randn((T, H), generator=g2).to(torch.bfloat16).to(dev)
+                indices, weights = route_topk(torch.randn((T, E), generator=g2).to(dev), K)
+                passes.append(layer(x, indices, weights).clone())
+            torch.cuda.synchronize()
+            layer.check()
+            outs.append(torch.stack(passes))
+        finally:
+            layer.destroy()
+    assert outs[0].abs().max() > 0
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
+def test_layer_captured_behind_a_join_a_copy_and_a_memset() -> None:
+    """Launches that may overlap their predecessor, where that is no kernel or more than one: work of
+    another stream that the captured stream waits for, a copy and a memset."""
+    from pplx_garden.models import ExpertParallelMoE, route_topk
+
+    dev = torch.device("cuda", 0)
+    H, I, E, K, T = 512, 256, 8, 2, 40
+    layer = ExpertParallelMoE(hidden_dim=H, intermediate_dim=I, num_experts=E, num_experts_per_token=K,
+                              max_num_tokens=T, device=dev, global_group=None, init_std=0.05)
+    try:
+        gen = torch.Generator(device="cpu").manual_seed(3)
+        x_in, logits_in = torch.randn((T, H), generator=gen).to(torch.bfloat16).to(dev), torch.randn((T, E), generator=gen).to(dev)
+        x, logits, out = torch.zeros_like(x_in), torch.zeros_like(logits_in), torch.zeros_like(x_in)
+        stream, side = torch.cuda.Stream(device=dev), torch.cuda.Stream(device=dev)
+
+        def step() -> None:
+            main = torch.cuda.current_stream()
+            side.wait_stream(main)
+            with torch.cuda.stream(side):
+                x.copy_(x_in)
+            logits.copy_(logits_in)
+            main.wait_stream(side)                       # a join ...
+            indices, weights = route_topk(logits, K)     # ... in front of the router
+            out.zero_()                                  # a memset in front of dispatch
+            layer(x, indices, weights, out=out)
+            side.wait_stream(main)
+            with torch.cuda.stream(side):
+                x.zero_()                                # after the layer has read it
+            main.wait_stream(side)
+
+        with torch.cuda.stream(stream):
+            step()
+        stream.synchronize()
+        want = out.clone()
+        assert want.abs().max() > 0
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.stream(stream):
+            with torch.cuda.graph(graph, stream=stream):
+                step()
+            for factor in (1.0, 2.0, 1.0):
+                x_in.mul_(factor)
+                out.fill_(9)
+                graph.replay()
+                if factor != 1.0:
+                    x_in.div_(factor)
+            stream.synchronize()
+        assert torch.equal(out, want)
+        layer.check()
+    finally:
+        layer.destroy()
