@@ -21,14 +21,14 @@ namespace {
 uint32_t round_up_u32(uint32_t a, uint32_t b) { return (a + b - 1) / b * b; }
 
 // A kernel stays loaded for the life of the process: every later context on the device finds it there.
-void preload_once(const A2AConfig& cfg, int out_dtype, int device, bool single) {
+void preload_once(const A2AConfig& cfg, int device, bool single) {
   static std::mutex mu;
-  static std::set<std::tuple<int, int, bool, int, int, int>> loaded;
+  static std::set<std::tuple<int, int, bool>> loaded;
   std::lock_guard<std::mutex> lock(mu);
-  const auto key = std::make_tuple(device, cfg.wire, single, cfg.in_elemsize, cfg.out_elemsize, out_dtype);
+  const auto key = std::make_tuple(device, cfg.wire, single);
   if (loaded.count(key) != 0) return;
-  PPLX_CUDA_CHECK(a2a_preload_kernels(cfg, out_dtype));
-  if (single) PPLX_CUDA_CHECK(a2a_preload_single(cfg, out_dtype));
+  PPLX_CUDA_CHECK(a2a_preload_kernels(cfg));
+  if (single) PPLX_CUDA_CHECK(a2a_preload_single());
   loaded.insert(key);
 }
 
@@ -184,7 +184,7 @@ A2AContext::A2AContext(const A2AParams& params, int device, const std::vector<in
 
   const char* trace_env = std::getenv("PPLX_A2A_TRACE");
   cfg_.trace = (trace_env != nullptr && std::atoi(trace_env) != 0) ? 1 : 0;
-  preload_once(cfg_, params.out_dtype, device_, single_rank());
+  preload_once(cfg_, device_, single_rank());
   const char* team_env = std::getenv("PPLX_A2A_TEAM");
   if (team_env != nullptr) team_override_ = std::atoi(team_env);
 

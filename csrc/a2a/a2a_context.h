@@ -30,7 +30,6 @@ struct A2AParams {
   int hidden_dim_scale = 0;
   int in_elemsize = 2;
   int out_elemsize = 2;
-  int out_dtype = kDtypeBF16;  // of the combined tokens
   int scale_elemsize = 4;
   int expert_padding = 1;
   int combine_mode = kCombinePerRoute;

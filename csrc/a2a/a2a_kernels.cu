@@ -1174,30 +1174,34 @@ cudaError_t a2a_launch_dispatch(const A2AConfig& cfg, const A2ARankStates& state
 
 namespace {
 template <int WIRE>
-cudaError_t preload_wire(int y_size, int out_dtype) {
+cudaError_t preload_wire() {
   cudaFuncAttributes attr;
   cudaError_t e = cudaFuncGetAttributes(&attr, dispatch_kernel<WIRE>);
-  for (int y : {kDtypeBF16, kDtypeF16, kDtypeF32}) {
-    if (e != cudaSuccess) return e;
+  if (e != cudaSuccess) return e;
+  const int dtypes[] = {kDtypeBF16, kDtypeF16, kDtypeF32};
+  for (int y : dtypes) {
     e = with_dtype(y, [&](auto* yp) {
       using Y = std::remove_pointer_t<decltype(yp)>;
-      if (sizeof(Y) != static_cast<size_t>(y_size)) return cudaSuccess;
-      const cudaError_t r = cudaFuncGetAttributes(&attr, combine_send_kernel<WIRE, Y>);
-      if (r != cudaSuccess) return r;
-      return with_dtype(out_dtype, [&](auto* op) {
-        using O = std::remove_pointer_t<decltype(op)>;
-        const cudaError_t q = cudaFuncGetAttributes(&attr, combine_kernel<WIRE, Y, O>);
-        return q != cudaSuccess ? q : cudaFuncGetAttributes(&attr, combine_recv_kernel<WIRE, Y, O>);
-      });
+      cudaError_t r = cudaFuncGetAttributes(&attr, combine_send_kernel<WIRE, Y>);
+      for (int o : dtypes) {
+        if (r != cudaSuccess) break;
+        r = with_dtype(o, [&](auto* op) {
+          using O = std::remove_pointer_t<decltype(op)>;
+          cudaError_t q = cudaFuncGetAttributes(&attr, combine_kernel<WIRE, Y, O>);
+          if (q == cudaSuccess) q = cudaFuncGetAttributes(&attr, combine_recv_kernel<WIRE, Y, O>);
+          return q;
+        });
+      }
+      return r;
     });
+    if (e != cudaSuccess) return e;
   }
-  return e != cudaSuccess ? e : cudaFuncGetAttributes(&attr, barrier_kernel);
+  return cudaFuncGetAttributes(&attr, barrier_kernel);
 }
 }  // namespace
 
-cudaError_t a2a_preload_kernels(const A2AConfig& cfg, int out_dtype) {
-  return cfg.wire == kWireLL ? preload_wire<kWireLL>(cfg.out_elemsize, out_dtype)
-                             : preload_wire<kWirePlain>(cfg.out_elemsize, out_dtype);
+cudaError_t a2a_preload_kernels(const A2AConfig& cfg) {
+  return cfg.wire == kWireLL ? preload_wire<kWireLL>() : preload_wire<kWirePlain>();
 }
 
 cudaError_t a2a_launch_barrier(const A2AConfig& cfg, const A2ARankStates& states, int nranks,

@@ -20,12 +20,11 @@ cudaError_t a2a_launch_dispatch(const A2AConfig& cfg, const A2ARankStates& state
                                 const PerRank<DispatchRecvArgs>& recv, int send_team, int recv_team,
                                 cudaStream_t stream);
 
-// Loads every kernel a context with this configuration can launch, on the current device: rows of
-// cfg.out_elemsize bytes an element, tokens of `out_dtype` (both are fixed for its life). With
+// Loads every kernel a context with this configuration can launch, on the current device. With
 // lazy module loading the first launch of a kernel may have to wait for the kernels that are
 // running; a dispatch that is running may in turn be waiting for a peer whose next kernel is
 // that first launch. Loading at set-up time takes the first launches out of the steady state.
-cudaError_t a2a_preload_kernels(const A2AConfig& cfg, int out_dtype);
+cudaError_t a2a_preload_kernels(const A2AConfig& cfg);
 
 // All ranks of the context meet on the device (bounded wait, reported through the status word).
 cudaError_t a2a_launch_barrier(const A2AConfig& cfg, const A2ARankStates& states, int nranks,
@@ -46,6 +45,6 @@ cudaError_t a2a_launch_dispatch_single(const A2AConfig& cfg, const A2ALocal& ws,
 cudaError_t a2a_launch_combine_single(const A2AConfig& cfg, const A2ALocal& ws, const CombineRecvArgs& recv,
                                       const uint8_t* rows, uint64_t row_stride, const uint32_t* arrived, int y_dtype,
                                       int out_dtype, cudaStream_t stream);
-cudaError_t a2a_preload_single(const A2AConfig& cfg, int out_dtype);
+cudaError_t a2a_preload_single();
 
 }  // namespace pplx

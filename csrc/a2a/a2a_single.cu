@@ -695,23 +695,22 @@ cudaError_t a2a_launch_combine_single(const A2AConfig& cfg, const A2ALocal& ws, 
   });
 }
 
-cudaError_t a2a_preload_single(const A2AConfig& cfg, int out_dtype) {
+cudaError_t a2a_preload_single() {
   cudaFuncAttributes attr;
-  cudaError_t e = cudaFuncGetAttributes(&attr, dispatch_single_kernel<true, false>);
+  cudaError_t e = cudaFuncGetAttributes(&attr, dispatch_single_kernel<true, true>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, dispatch_single_kernel<false, true>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, dispatch_single_kernel<true, false>);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, dispatch_single_kernel<false, false>);
-  if (cfg.in_elemsize == 1) {   // only such a wire type can be quantised to
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, dispatch_single_kernel<true, true>);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, dispatch_single_kernel<false, true>);
-  }
   for (int y : {kDtypeBF16, kDtypeF16, kDtypeF32}) {
-    if (e != cudaSuccess) return e;
-    e = with_types(y, out_dtype, [&](auto* yp, auto* op) {
-      using Y = std::remove_pointer_t<decltype(yp)>;
-      using O = std::remove_pointer_t<decltype(op)>;
-      if (sizeof(Y) != static_cast<size_t>(cfg.out_elemsize)) return cudaSuccess;
-      const cudaError_t q = cudaFuncGetAttributes(&attr, combine_bulk_kernel<Y, O>);
-      return q != cudaSuccess ? q : cudaFuncGetAttributes(&attr, combine_single_kernel<Y, O>);
-    });
+    for (int o : {kDtypeBF16, kDtypeF16, kDtypeF32}) {
+      if (e != cudaSuccess) return e;
+      e = with_types(y, o, [&](auto* yp, auto* op) {
+        using Y = std::remove_pointer_t<decltype(yp)>;
+        using O = std::remove_pointer_t<decltype(op)>;
+        const cudaError_t q = cudaFuncGetAttributes(&attr, combine_bulk_kernel<Y, O>);
+        return q != cudaSuccess ? q : cudaFuncGetAttributes(&attr, combine_single_kernel<Y, O>);
+      });
+    }
   }
   return e;
 }

@@ -323,12 +323,12 @@ void bind_a2a(py::module_& m) {
             } else {
               local_ranks = rank.cast<std::vector<int>>();
             }
-            A2AParams p = make_params(hidden_dim, hidden_dim_scale, in_elemsize, out_elemsize,
-                                      scale_elemsize, max_num_tokens, num_experts,
-                                      expert_padding, num_experts_per_token, dp_size,
-                                      world_size, combine_mode, num_blocks, wait_limit_ms, wire, node_mask);
+            const A2AParams p = make_params(hidden_dim, hidden_dim_scale, in_elemsize, out_elemsize,
+                                            scale_elemsize, max_num_tokens, num_experts,
+                                            expert_padding, num_experts_per_token, dp_size,
+                                            world_size, combine_mode, num_blocks, wait_limit_ms, wire, node_mask);
             auto self = std::make_unique<PyA2A>();
-            self->out_dtype = p.out_dtype = dtype_code(out_dtype);
+            self->out_dtype = dtype_code(out_dtype);
             self->ctx = std::make_unique<A2AContext>(p, device, local_ranks,
                                                      ptr_tables(sync_ptrs, local_ranks.size()),
                                                      ptr_tables(recv_ptrs, local_ranks.size()));
