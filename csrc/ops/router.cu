@@ -19,6 +19,7 @@
 
 #include <algorithm>
 #include <cfloat>
+#include <cmath>
 
 #include "../a2a/ptx.cuh"
 #include "../core/error.h"
@@ -214,6 +215,31 @@ __global__ void __launch_bounds__(kMaxWarps * 32, kBlocksPerSm<PER_LANE>) topk_r
   }
 }
 
+template <int PER_LANE>
+__global__ void __launch_bounds__(kMaxWarps * 32) topk_rounds_kernel(const __grid_constant__ TopkRouteParams p) {
+  grid_wait();
+  grid_allow_next();
+  const int tokens = p.bound != nullptr ? min(p.tokens, *p.bound) : p.tokens;
+  const int token = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (token < tokens) route_by_rounds<PER_LANE>(p, token, threadIdx.x & 31);
+}
+
+// Whether the rounds alone beat the ranking. Its candidates have to fit 32 places: with L lanes that hold
+// PER_LANE keys each, a bound that k + 1 of their maxima reach lets through about
+// E (1 - (1 - (k + 1) / L)^(1 / PER_LANE)) keys, and from about 33 on a token does both more often than not.
+// 32,768 tokens, rounds and ranking in us: 256 experts k = 20 73 and 66, k = 24 85 and 102; 320 experts k = 14
+// 102 and 76, k = 16 114 and 130; 512 experts k = 18 135 and 87, k = 20 146 and 157. With four keys a lane or
+// fewer the ranking keeps up at any k (128 experts k = 32 84 and 75). One or two rounds are
+// shorter than the ranking's set-up where a lane holds four or eight keys (256 experts k = 1 16.2 and 17.7).
+template <int PER_LANE>
+bool rounds_win(int experts, int k, bool vec) {
+  if (k <= 2) return PER_LANE == 4 || PER_LANE == 8;
+  if (PER_LANE < 8 || k < 8) return false;
+  const double lanes = vec ? experts / PER_LANE : 32;
+  const double left = std::max(0.0, 1.0 - (k + 1) / lanes);
+  return experts * (1.0 - std::pow(left, 1.0 / PER_LANE)) > 33.0;
+}
+
 template <int PER_LANE, typename T>
 void launch(const TopkRouteParams& p, int sms, cudaStream_t stream) {
   constexpr uintptr_t kAlign = std::min<size_t>(16, PER_LANE * sizeof(T));
@@ -225,9 +251,12 @@ void launch(const TopkRouteParams& p, int sms, cudaStream_t stream) {
   // Few tokens: one warp a block, so that they spread over the SMs. Many: one wave of resident blocks
   // whose warps loop, with the bias in registers.
   const int warps = p.tokens <= sms * 4 ? 1 : kMaxWarps;
-  const int blocks = std::min((p.tokens + warps - 1) / warps, sms * (warps == 1 ? 4 : kBlocksPerSm<PER_LANE>));
-  const void* kernel = vec ? reinterpret_cast<const void*>(topk_route_kernel<PER_LANE, T, true>)
-                           : reinterpret_cast<const void*>(topk_route_kernel<PER_LANE, T, false>);
+  const int groups = (p.tokens + warps - 1) / warps;
+  const bool rounds = rounds_win<PER_LANE>(p.num_experts, p.k, vec);
+  const int blocks = rounds ? groups : std::min(groups, sms * (warps == 1 ? 4 : kBlocksPerSm<PER_LANE>));
+  const void* kernel = rounds ? reinterpret_cast<const void*>(topk_rounds_kernel<PER_LANE>)
+                       : vec  ? reinterpret_cast<const void*>(topk_route_kernel<PER_LANE, T, true>)
+                              : reinterpret_cast<const void*>(topk_route_kernel<PER_LANE, T, false>);
   void* args[] = {const_cast<TopkRouteParams*>(&p)};
   PPLX_CUDA_CHECK(launch_overlapped(kernel, dim3(blocks), dim3(warps * 32), args, 0, stream));
 }

@@ -113,3 +113,19 @@ def test_k_at_the_number_of_filled_lanes(experts, k):
     assert torch.equal(idx.view(torch.int32).cpu().long(), want)
     # __expf: 2 ulp and |x| ulp, |x| below 10 here
     assert torch.allclose(w.cpu(), torch.softmax(torch.gather(logits.cpu(), 1, want), dim=-1), rtol=1e-5, atol=1e-7)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("experts,ranked,rounds", [(128, 3, 2), (160, 14, 17), (256, 3, 1), (256, 19, 22), (320, 14, 16), (384, 16, 18),
+                                                   (512, 18, 21), (512, 3, 2), (1000, 19, 24), (1024, 8, 32)])
+@pytest.mark.parametrize("tokens", [9, 3000])
+def test_ranking_and_rounds_on_both_sides_of_their_rule(experts, ranked, rounds, tokens):
+    dev = torch.device("cuda", 0)
+    logits = torch.randn((tokens, experts), generator=torch.Generator().manual_seed(experts + ranked)).to(dev)
+    x = logits.cpu()
+    order = torch.sort(x, dim=-1, descending=True, stable=True).indices
+    for k in (ranked, rounds):
+        idx, w = topk_route(logits, k)
+        assert torch.equal(idx.view(torch.int32).cpu().long(), order[:, :k])
+        # __expf: 2 ulp and |x| ulp, |x| below 12 here
+        assert torch.allclose(w.cpu(), torch.softmax(torch.gather(x, 1, order[:, :k]), dim=-1), rtol=1e-5, atol=1e-7)
