@@ -79,12 +79,19 @@ __global__ void __launch_bounds__(kSingleThreads, 1) dispatch_single_kernel(cons
   __shared__ uint32_t s_rows[kBatchTokens * kMaxTopK];
   __shared__ uint32_t s_warp_sum[kSingleWarps];
   __shared__ uint64_t s_bars[kSingleWarps][2];
+  __shared__ uint32_t s_failed;
   const A2AConfig& cfg = d.cfg;
   const A2ALocal& ws = d.ws;
   const DispatchSendArgs& a = d.send;
   const DispatchRecvArgs& r = d.recv;
   grid_wait();
   grid_allow_next();
+  // One thread reads the status word for its block: block 0 of this very launch may write it (an expert
+  // that does not exist, rows that do not fit), and a block that starts late must not be of two minds. The
+  // block decides at its second barrier, when the word has come in anyway (128 tokens of 14 KiB: deciding
+  // at the first one costs 0.2 us).
+  uint32_t status = 0;
+  if (threadIdx.x == 0) status = *reinterpret_cast<volatile const uint32_t*>(&ws.status[0]);
   const uint32_t E = cfg.num_experts;
   const uint32_t K = cfg.topk;
   uint32_t* total = reinterpret_cast<uint32_t*>(dyn_smem + (kBulk ? kSingleWarps * 2 * kPieceBuffer : 0));
@@ -132,8 +139,8 @@ __global__ void __launch_bounds__(kSingleThreads, 1) dispatch_single_kernel(cons
     if constexpr (kQuant) piece = load_quantised(source(u), i, nvec, pow2, &piece_scale);
     else if (i < nvec) piece = ld_after_wait_v4(source(u) + 16ull * i);
   };
-  // Nor does the routing table's count depend on anything above: its first loads are under way while the
-  // status word comes in. They have to stand here: below, the barrier would hold them back.
+  // Nor does the count of the routing table, whose first loads stand here because the barrier below would
+  // hold them back.
   const uint32_t routes = static_cast<uint32_t>(T) * K;
   const bool vector_indices = a.indices_stride == K && (reinterpret_cast<uintptr_t>(a.indices) & 15u) == 0;
   const uint32_t quads = vector_indices ? routes / 4 : 0u;
@@ -147,13 +154,6 @@ __global__ void __launch_bounds__(kSingleThreads, 1) dispatch_single_kernel(cons
     }
   };
   load_quads(threadIdx.x);
-  if constexpr (!kBulk) {
-    if (unit < units) load(unit);
-  }
-  // One thread reads the status word for its block: block 0 of this very launch may write it (an expert
-  // that does not exist, rows that do not fit), and a block that starts late must not be of two minds.
-  __shared__ uint32_t s_failed;
-  if (threadIdx.x == 0) s_failed = *reinterpret_cast<volatile const uint32_t*>(&ws.status[0]);
   if constexpr (kBulk && !kQuant) {
     if (lane == 0) {
       mbar_init(&s_bars[warp][0], 1);
@@ -161,14 +161,12 @@ __global__ void __launch_bounds__(kSingleThreads, 1) dispatch_single_kernel(cons
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncwarp();
+    fetch(unit, 0);
+  } else if constexpr (!kBulk) {
+    if (unit < units) load(unit);
   }
   for (uint32_t i = threadIdx.x; i < 2 * E; i += kSingleThreads) total[i] = 0;
   __syncthreads();
-  if (s_failed != 0) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) ws.single_done[0] += 1;
-    return;
-  }
-  if constexpr (kBulk && !kQuant) fetch(unit, 0);
   // ---- routes per expert, those of earlier blocks' tokens apart ----
   auto count = [&](uint32_t e, bool earlier, uint32_t t) {
     if (e < E) atomicAdd(earlier ? &next[e] : &total[e], 1u);
@@ -195,7 +193,15 @@ __global__ void __launch_bounds__(kSingleThreads, 1) dispatch_single_kernel(cons
       count(a.indices[t * a.indices_stride + i % K], t < t0, t);
     }
   }
+  if (threadIdx.x == 0) s_failed = status;
   __syncthreads();
+  if (s_failed != 0) {
+    if constexpr (kBulk && !kQuant) {   // no copy may still be on its way into a block that has left
+      if (lane == 0 && unit < units) mbar_wait_timed(&s_bars[warp][0], 0, cfg.wait_limit_ns);
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) ws.single_done[0] += 1;
+    return;
+  }
   // ---- expert-major layout: exclusive scan of the padded totals, kSingleThreads experts at a time ----
   const uint32_t pad = cfg.expert_padding;
   const uint32_t row_cap = r.out_rows ? min(r.out_rows, cfg.max_recv_rows) : cfg.max_recv_rows;
@@ -370,25 +376,24 @@ struct SingleCombine {
   uint32_t segment;           // combine_bulk_kernel: bytes of each row that a warp reduces at a time
 };
 
-// Whether the rows may be reduced; called by all threads of every block, before any of them is read. One
-// thread decides for its block, as in dispatch: the status word may change while the block looks at it.
-__device__ __forceinline__ bool combine_ready(const SingleCombine& c) {
+// Whether the rows may be reduced; called by all threads of every block, before any of them is read. All
+// lanes of a warp get the same answer: the status word may change while they look at it.
+__device__ __forceinline__ bool combine_ready(const SingleCombine& c, uint32_t status) {
   const A2ALocal& ws = c.ws;
-  __shared__ uint32_t s_go;
-  if (threadIdx.x == 0) {
-    bool go = *reinterpret_cast<volatile const uint32_t*>(&ws.status[0]) == 0;
-    if (c.recv.external) {
+  bool go = status == 0;
+  if (c.recv.external) {
+    __shared__ uint32_t s_arrived;
+    if (threadIdx.x == 0) {
       const uint32_t expected = read_epoch(ws, 2) + 1;
       uint64_t waited;
-      const bool arrived = wait_flag(c.arrived, expected, c.cfg.wait_limit_ns, &waited);
-      if (!arrived) report(ws, kStatusWaitTimeout, kPhaseCombineRecv, 0, expected);
+      s_arrived = wait_flag(c.arrived, expected, c.cfg.wait_limit_ns, &waited) ? 1u : 0u;
+      if (!s_arrived) report(ws, kStatusWaitTimeout, kPhaseCombineRecv, 0, expected);
       if (blockIdx.x == 0) atomicMax(&ws.stats[3], static_cast<unsigned long long>(waited));
-      go = go && arrived;
     }
-    s_go = go ? 1u : 0u;
+    __syncthreads();
+    go = go && s_arrived != 0;
   }
-  __syncthreads();
-  return s_go != 0;
+  return __all_sync(0xffffffffu, go);
 }
 
 __device__ __forceinline__ void combine_finish(const SingleCombine& c, uint32_t epoch) {
@@ -399,32 +404,38 @@ __device__ __forceinline__ void combine_finish(const SingleCombine& c, uint32_t 
   }
 }
 
-// Lane k: where token t's k-th row is (kNoSlot: nowhere) and its weight. All 32 lanes call. The routes of
-// the combine decide what is reduced, as in the general kernels: one with an expert that does not exist
-// is left out (in the pre-reduced mode only a token with no other counts for nothing), so that a
-// caller may dispatch by bound_m and combine the padding too, or mask single routes. `dispatched`: tokens
-// that were; the rows of a later one never come.
-__device__ __forceinline__ void combine_route(const SingleCombine& c, uint32_t t, uint32_t lane, uint32_t dispatched,
-                                              uint32_t* row, float* w) {
+// Lane k: where token t's k-th row is and its weight. The routes of the combine decide what is reduced, as
+// in the general kernels: one with an expert that does not exist is left out (in the pre-reduced mode
+// only a token that has no other), so that a caller may dispatch by bound_m and combine the padding too, or
+// mask single routes. Loaded by one call and judged by another, so that nothing waits for the loads
+// in between (judged at once, 4096 tokens of 8 rows of 14 KiB took 25 us more).
+struct Route {
+  uint32_t row = kNoSlot, expert = ~0u;
+  uint32_t dispatched = 0;   // tokens that were: the rows of a later one never come
+  float w = 0.f;
+};
+__device__ __forceinline__ Route load_route(const SingleCombine& c, uint32_t t, uint32_t lane) {
   const A2AConfig& cfg = c.cfg;
   const CombineRecvArgs& a = c.recv;
   const uint32_t K = cfg.topk;
-  const bool per_route = cfg.combine_mode == kCombinePerRoute;
-  *row = kNoSlot;
-  *w = 0.f;
-  bool valid = false;
+  Route r;
+  r.dispatched = c.ws.expert_meta[1];
   if (lane < K) {
     const uint64_t tk = static_cast<uint64_t>(t) * K + lane;
-    valid = a.indices[t * a.indices_stride + lane] < static_cast<uint32_t>(cfg.num_experts);
-    if (a.external) *row = static_cast<uint32_t>(tk);
-    else if (t < dispatched) *row = c.ws.route_row[tk];
-    *w = a.external || per_route ? a.weights[t * a.weights_stride + lane] : c.ws.rec_weights[tk];
+    r.expert = a.indices[t * a.indices_stride + lane];
+    r.row = a.external ? static_cast<uint32_t>(tk) : c.ws.route_row[tk];
+    r.w = a.external || cfg.combine_mode == kCombinePerRoute ? a.weights[t * a.weights_stride + lane] : c.ws.rec_weights[tk];
   }
-  const uint32_t any = __ballot_sync(0xffffffffu, valid);
-  if (per_route ? !valid : any == 0) *row = kNoSlot;
-  if (!a.external && t >= dispatched && any != 0 && lane == 0) {
-    report(c.ws, kStatusWaitTimeout, kPhaseCombineRecv, t, dispatched);
-  }
+  return r;
+}
+// The row, or kNoSlot. All 32 lanes call.
+__device__ __forceinline__ uint32_t route_place(const SingleCombine& c, const Route& r, uint32_t t) {
+  const bool valid = r.expert < static_cast<uint32_t>(c.cfg.num_experts);
+  if (c.cfg.combine_mode == kCombinePerRoute && (c.recv.external || t < r.dispatched)) return valid ? r.row : kNoSlot;
+  const bool any = __any_sync(0xffffffffu, valid);
+  if (t < r.dispatched) return any ? r.row : kNoSlot;
+  if (any && (threadIdx.x & 31u) == 0) report(c.ws, kStatusWaitTimeout, kPhaseCombineRecv, t, r.dispatched);
+  return kNoSlot;   // the table holds an earlier dispatch's
 }
 
 // acc += w_k * row_k over the rows of `have` (bit k: row k is there), 16 bytes of each, at `p` and every
@@ -477,7 +488,7 @@ __global__ void __launch_bounds__(kBulkWarps * 32, 1) combine_bulk_kernel(const 
   grid_allow_next();
   const uint32_t T = bounded_tokens(cfg, a.num_tokens, a.bound_m);
   const uint32_t epoch = a.external ? read_epoch(c.ws, 1) : 0u;
-  const uint32_t dispatched = c.ws.expert_meta[1];
+  const uint32_t status = *reinterpret_cast<volatile const uint32_t*>(&c.ws.status[0]);
   uint64_t* const bars = s_bars[warp];
   if (lane == 0) {
     mbar_init(&bars[0], 1);
@@ -493,20 +504,16 @@ __global__ void __launch_bounds__(kBulkWarps * 32, 1) combine_bulk_kernel(const 
   const uint32_t step = gridDim.x * kBulkWarps;
   // Routes are fetched one job before the rows, rows one job before they are reduced.
   uint32_t job = blockIdx.x * kBulkWarps + warp;   // the warps of a block work on neighbouring pieces
-  uint32_t row, next_row;
-  float w, next_w;
-  auto route = [&](uint32_t j, uint32_t* r, float* wt) {
-    *r = kNoSlot;
-    *wt = 0.f;
-    if (j < jobs) combine_route(c, j / pieces, lane, dispatched, r, wt);
-  };
-  route(job, &row, &w);
-  if (combine_ready(c)) {
+  auto route = [&](uint32_t j) { return j < jobs ? load_route(c, j / pieces, lane) : Route(); };
+  const Route first = route(job);
+  if (combine_ready(c, status)) {
     // rows of a kernel that is still running on another stream: written by plain stores that the
     // arrival counter covers, read by the bulk-copy engine below
     if (a.external) asm volatile("fence.proxy.async;" ::: "memory");
     uint8_t* const buffers = dyn_smem + warp * 2 * kBulkBuffer;
-    auto fetch = [&](uint32_t j, uint32_t r, uint32_t slot) -> uint32_t {   // returns which rows come
+    auto fetch = [&](uint32_t j, const Route& route, uint32_t slot) -> uint32_t {   // returns which rows come
+      if (j >= jobs) return 0;
+      const uint32_t r = route_place(c, route, j / pieces);
       const uint32_t have = __ballot_sync(0xffffffffu, r != kNoSlot);
       if (have != 0) {
         const uint32_t off = j % pieces * seg;
@@ -520,14 +527,13 @@ __global__ void __launch_bounds__(kBulkWarps * 32, 1) combine_bulk_kernel(const 
       }
       return have;
     };
-    uint32_t have = fetch(job, row, 0);
-    route(job + step, &next_row, &next_w);
+    uint32_t have = fetch(job, first, 0);
+    float w = first.w;
+    Route next = route(job + step);
     uint32_t slot = 0, parities = 0;
     for (; job < jobs; job += step) {
-      const uint32_t next_have = fetch(job + step, next_row, slot ^ 1u);   // no rows past the last job
-      uint32_t after_row;
-      float after_w;
-      route(job + 2 * step, &after_row, &after_w);
+      const uint32_t next_have = fetch(job + step, next, slot ^ 1u);   // no rows past the last job
+      const Route after = route(job + 2 * step);
       const uint32_t t = job / pieces, off = job % pieces * seg;
       const uint32_t bytes = min(seg, row_bytes - off);
       if (have != 0) {
@@ -548,9 +554,8 @@ __global__ void __launch_bounds__(kBulkWarps * 32, 1) combine_bulk_kernel(const 
       }
       __syncwarp();   // the buffer is filled again
       have = next_have;
-      w = next_w;
-      next_row = after_row;
-      next_w = after_w;
+      w = next.w;
+      next = after;
       slot ^= 1u;
     }
   }
@@ -568,20 +573,25 @@ __global__ void __launch_bounds__(kCombineThreads, 1) combine_single_kernel(cons
   grid_allow_next();
   const int T = bounded_tokens(cfg, a.num_tokens, a.bound_m);
   const uint32_t epoch = a.external ? read_epoch(ws, 1) : 0u;
-  const uint32_t dispatched = ws.expert_meta[1];
+  const uint32_t status = *reinterpret_cast<volatile const uint32_t*>(&ws.status[0]);
   const uint32_t ngran = cfg.hidden_dim / 8;
   const uint32_t pieces = (ngran + 31) / 32;
   constexpr int kVecs = Elem8<Y>::kBytes / 16;
   constexpr int U = 8 / kVecs;   // rows in flight per lane
   const uint32_t warps = gridDim.x * kCombineWarps;
   const uint32_t first = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-  uint32_t my_row = kNoSlot;   // the first unit's routes come in while the block makes up its mind
+  uint32_t my_row = kNoSlot;   // the first unit's come in with the status word
   float my_w = 0.f;
-  if (first < T * pieces) combine_route(c, first / pieces, lane, dispatched, &my_row, &my_w);
-  if (combine_ready(c)) {
+  auto route = [&](uint32_t t) {
+    const Route r = load_route(c, t, lane);
+    my_row = route_place(c, r, t);
+    my_w = r.w;
+  };
+  if (first < T * pieces) route(first / pieces);
+  if (combine_ready(c, status)) {
     for (uint32_t unit = first; unit < T * pieces; unit += warps) {
       const uint32_t t = unit / pieces;
-      if (unit != first) combine_route(c, t, lane, dispatched, &my_row, &my_w);
+      if (unit != first) route(t);
       uint8_t* out_row = a.out_tokens + static_cast<uint64_t>(t) * a.out_tokens_stride * sizeof(O);
       const uint32_t g = unit % pieces * 32 + lane;
       const bool inside = g < ngran;
