@@ -145,11 +145,10 @@ __global__ void __launch_bounds__(kMaxWarps * 32, kBlocksPerSm<PER_LANE>) topk_r
     // At least k lanes have best >= lo, fewer than k have best >= hi. Lanes whose run of experts lies past
     // the last one hold no key and are left out: with them in, the minimum is 0 and everything is a
     // candidate (160 experts fill 20 lanes of 8: 32,768 tokens took 37 us, and 29 by rounds alone).
-    const int holding = __popc(__ballot_sync(0xffffffffu, best != 0));
-    uint32_t lo = __reduce_min_sync(0xffffffffu, best != 0 ? best : 0xffffffffu);
+    uint32_t lo = __reduce_min_sync(0xffffffffu, best - 1u) + 1u;   // no key, 0, is the largest here
     uint32_t hi = __reduce_max_sync(0xffffffffu, best);
-    if (holding >= k) {
-      int have = holding;
+    if (E > 32) {
+      int have = kVec ? E / PER_LANE : 32;   // lanes with a key: k at least, see launch()
       for (int step = 0; step < 12 && have > k + 2 && hi - lo > 1; ++step) {
         const uint32_t mid = lo + (hi - lo) / 2;
         const int n = __popc(__ballot_sync(0xffffffffu, best >= mid));
@@ -161,7 +160,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, kBlocksPerSm<PER_LANE>) topk_r
         }
       }
     } else {
-      lo = 0;   // 32 experts or fewer (see launch()): all of them are candidates
+      lo = 0;   // all of them are candidates
     }
     const uint32_t bound = max(lo, 1u);
     // the candidates' places in the scratch: any order will do
@@ -221,15 +220,25 @@ __global__ void __launch_bounds__(kMaxWarps * 32) topk_rounds_kernel(const __gri
   grid_allow_next();
   const int tokens = p.bound != nullptr ? min(p.tokens, *p.bound) : p.tokens;
   const int token = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (token < tokens) route_by_rounds<PER_LANE>(p, token, threadIdx.x & 31);
+  if (token >= tokens) return;
+  const int lane = threadIdx.x & 31;
+  uint32_t idx;
+  float weight;
+  route_token_warp<PER_LANE>(static_cast<const char*>(p.logits) + static_cast<int64_t>(token) * p.logits_stride * (p.logits_bf16 ? 2 : 4),
+                             p.logits_bf16, p.bias, p.num_experts, p.k, &idx, &weight);
+  if (lane < p.k) {
+    p.indices[token * p.indices_stride + lane] = idx;
+    p.weights[token * p.weights_stride + lane] = weight;
+  }
 }
 
 // Whether the rounds alone beat the ranking. Its candidates have to fit 32 places: with L lanes that hold
-// PER_LANE keys each, a bound that k + 1 of their maxima reach lets through about
-// E (1 - (1 - (k + 1) / L)^(1 / PER_LANE)) keys, and from about 33 on a token does both more often than not.
-// 32,768 tokens, rounds and ranking in us: 256 experts k = 20 73 and 66, k = 24 85 and 102; 320 experts k = 14
-// 102 and 76, k = 16 114 and 130; 512 experts k = 18 135 and 87, k = 20 146 and 157. With four keys a lane or
-// fewer the ranking keeps up at any k (128 experts k = 32 84 and 75). One or two rounds are
+// E / L keys each, a bound that k + 1 of their maxima reach lets through about
+// E (1 - (1 - (k + 1) / L)^(L / E)) keys. From about 33 on a token does both more often than not; with more
+// than 16 keys a lane, whose rounds are long, ranking pays up to 36. 32,768 tokens, rounds and ranking in us:
+// 256 experts k = 20 73 and 66, k = 24 85 and 102; 320 experts k = 14 102 and 76, k = 16 114 and 130; 512
+// experts k = 18 135 and 87, k = 20 146 and 157; 1000 experts k = 20 335 and 304, k = 24 379 and 428. With four
+// keys a lane or fewer the ranking keeps up at any k (128 experts k = 32 84 and 75). One or two rounds are
 // shorter than the ranking's set-up where a lane holds four or eight keys (256 experts k = 1 16.2 and 17.7).
 template <int PER_LANE>
 bool rounds_win(int experts, int k, bool vec) {
@@ -237,7 +246,7 @@ bool rounds_win(int experts, int k, bool vec) {
   if (PER_LANE < 8 || k < 8) return false;
   const double lanes = vec ? experts / PER_LANE : 32;
   const double left = std::max(0.0, 1.0 - (k + 1) / lanes);
-  return experts * (1.0 - std::pow(left, 1.0 / PER_LANE)) > 33.0;
+  return experts * (1.0 - std::pow(left, lanes / experts)) > (PER_LANE > 16 ? 36.0 : 33.0);
 }
 
 template <int PER_LANE, typename T>
