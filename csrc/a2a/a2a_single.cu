@@ -84,14 +84,6 @@ __global__ void __launch_bounds__(kSingleThreads, 1) dispatch_single_kernel(cons
   const A2ALocal& ws = d.ws;
   const DispatchSendArgs& a = d.send;
   const DispatchRecvArgs& r = d.recv;
-  grid_wait();
-  grid_allow_next();
-  // One thread reads the status word for its block: block 0 of this very launch may write it (an expert
-  // that does not exist, rows that do not fit), and a block that starts late must not be of two minds. The
-  // block decides at its second barrier, when the word has come in anyway (128 tokens of 14 KiB: deciding
-  // at the first one costs 0.2 us).
-  uint32_t status = 0;
-  if (threadIdx.x == 0) status = *reinterpret_cast<volatile const uint32_t*>(&ws.status[0]);
   const uint32_t E = cfg.num_experts;
   const uint32_t K = cfg.topk;
   uint32_t* total = reinterpret_cast<uint32_t*>(dyn_smem + (kBulk ? kSingleWarps * 2 * kPieceBuffer : 0));
@@ -99,6 +91,24 @@ __global__ void __launch_bounds__(kSingleThreads, 1) dispatch_single_kernel(cons
   // total: [E] routes of tokens from t0 on; next: [E] routes of tokens before t0, then the next free row
   const int warp = threadIdx.x >> 5;
   const uint32_t lane = threadIdx.x & 31u;
+  // shared memory only: this may run under the end of the kernel before
+  for (uint32_t i = threadIdx.x; i < 2 * E; i += kSingleThreads) total[i] = 0;
+  if constexpr (kBulk && !kQuant) {
+    if (lane == 0) {
+      mbar_init(&s_bars[warp][0], 1);
+      mbar_init(&s_bars[warp][1], 1);
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+  }
+  __syncthreads();
+  grid_wait();
+  grid_allow_next();
+  // One thread reads the status word for its block: block 0 of this very launch may write it (an expert
+  // that does not exist, rows that do not fit), and a block that starts late must not be of two minds. The
+  // block decides after the count, when the word has come in anyway (128 tokens of 14 KiB: waiting for it
+  // before costs 0.2 us).
+  uint32_t status = 0;
+  if (threadIdx.x == 0) status = *reinterpret_cast<volatile const uint32_t*>(&ws.status[0]);
   const uint32_t nvec = cfg.d_payload_bytes / 16;
   constexpr uint32_t kPieceVecs = kBulk ? kPieceBytes / 16 : 32;
   const uint32_t chunks = (nvec + kPieceVecs - 1) / kPieceVecs;
@@ -139,8 +149,6 @@ __global__ void __launch_bounds__(kSingleThreads, 1) dispatch_single_kernel(cons
     if constexpr (kQuant) piece = load_quantised(source(u), i, nvec, pow2, &piece_scale);
     else if (i < nvec) piece = ld_after_wait_v4(source(u) + 16ull * i);
   };
-  // Nor does the count of the routing table, whose first loads stand here because the barrier below would
-  // hold them back.
   const uint32_t routes = static_cast<uint32_t>(T) * K;
   const bool vector_indices = a.indices_stride == K && (reinterpret_cast<uintptr_t>(a.indices) & 15u) == 0;
   const uint32_t quads = vector_indices ? routes / 4 : 0u;
@@ -155,18 +163,10 @@ __global__ void __launch_bounds__(kSingleThreads, 1) dispatch_single_kernel(cons
   };
   load_quads(threadIdx.x);
   if constexpr (kBulk && !kQuant) {
-    if (lane == 0) {
-      mbar_init(&s_bars[warp][0], 1);
-      mbar_init(&s_bars[warp][1], 1);
-      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncwarp();
     fetch(unit, 0);
   } else if constexpr (!kBulk) {
     if (unit < units) load(unit);
   }
-  for (uint32_t i = threadIdx.x; i < 2 * E; i += kSingleThreads) total[i] = 0;
-  __syncthreads();
   // ---- routes per expert, those of earlier blocks' tokens apart ----
   auto count = [&](uint32_t e, bool earlier, uint32_t t) {
     if (e < E) atomicAdd(earlier ? &next[e] : &total[e], 1u);
@@ -376,24 +376,22 @@ struct SingleCombine {
   uint32_t segment;           // combine_bulk_kernel: bytes of each row that a warp reduces at a time
 };
 
-// Whether the rows may be reduced; called by all threads of every block, before any of them is read. All
-// lanes of a warp get the same answer: the status word may change while they look at it.
-__device__ __forceinline__ bool combine_ready(const SingleCombine& c, uint32_t status) {
+// Called by all threads of every block, before any row is read: the status word, or something else than 0
+// where the rows of another kernel do not come. It may change while a warp's lanes look at it: they vote.
+__device__ __forceinline__ uint32_t combine_status(const SingleCombine& c) {
   const A2ALocal& ws = c.ws;
-  bool go = status == 0;
-  if (c.recv.external) {
-    __shared__ uint32_t s_arrived;
-    if (threadIdx.x == 0) {
-      const uint32_t expected = read_epoch(ws, 2) + 1;
-      uint64_t waited;
-      s_arrived = wait_flag(c.arrived, expected, c.cfg.wait_limit_ns, &waited) ? 1u : 0u;
-      if (!s_arrived) report(ws, kStatusWaitTimeout, kPhaseCombineRecv, 0, expected);
-      if (blockIdx.x == 0) atomicMax(&ws.stats[3], static_cast<unsigned long long>(waited));
-    }
-    __syncthreads();
-    go = go && s_arrived != 0;
+  const uint32_t status = *reinterpret_cast<volatile const uint32_t*>(&ws.status[0]);
+  if (!c.recv.external) return status;
+  __shared__ uint32_t s_arrived;
+  if (threadIdx.x == 0) {
+    const uint32_t expected = read_epoch(ws, 2) + 1;
+    uint64_t waited;
+    s_arrived = wait_flag(c.arrived, expected, c.cfg.wait_limit_ns, &waited) ? 1u : 0u;
+    if (!s_arrived) report(ws, kStatusWaitTimeout, kPhaseCombineRecv, 0, expected);
+    if (blockIdx.x == 0) atomicMax(&ws.stats[3], static_cast<unsigned long long>(waited));
   }
-  return __all_sync(0xffffffffu, go);
+  __syncthreads();
+  return s_arrived != 0 ? status : ~0u;
 }
 
 __device__ __forceinline__ void combine_finish(const SingleCombine& c, uint32_t epoch) {
@@ -408,10 +406,10 @@ __device__ __forceinline__ void combine_finish(const SingleCombine& c, uint32_t 
 // in the general kernels: one with an expert that does not exist is left out (in the pre-reduced mode
 // only a token that has no other), so that a caller may dispatch by bound_m and combine the padding too, or
 // mask single routes. Loaded by one call and judged by another, so that nothing waits for the loads
-// in between (judged at once, 4096 tokens of 8 rows of 14 KiB took 25 us more).
+// in between (judged at once, 4096 tokens of 8 rows of 14 KiB took 25 us more); all of them at once: as
+// plain loads the compiler moves them behind the first comparison.
 struct Route {
   uint32_t row = kNoSlot, expert = ~0u;
-  uint32_t dispatched = 0;   // tokens that were: the rows of a later one never come
   float w = 0.f;
 };
 __device__ __forceinline__ Route load_route(const SingleCombine& c, uint32_t t, uint32_t lane) {
@@ -419,23 +417,30 @@ __device__ __forceinline__ Route load_route(const SingleCombine& c, uint32_t t, 
   const CombineRecvArgs& a = c.recv;
   const uint32_t K = cfg.topk;
   Route r;
-  r.dispatched = c.ws.expert_meta[1];
   if (lane < K) {
     const uint64_t tk = static_cast<uint64_t>(t) * K + lane;
-    r.expert = a.indices[t * a.indices_stride + lane];
-    r.row = a.external ? static_cast<uint32_t>(tk) : c.ws.route_row[tk];
-    r.w = a.external || cfg.combine_mode == kCombinePerRoute ? a.weights[t * a.weights_stride + lane] : c.ws.rec_weights[tk];
+    const float* weight = a.external || cfg.combine_mode == kCombinePerRoute ? a.weights + t * a.weights_stride + lane
+                                                                             : c.ws.rec_weights + tk;
+    r.expert = ld_after_wait_u32(a.indices + t * a.indices_stride + lane);
+    r.row = a.external ? static_cast<uint32_t>(tk) : ld_after_wait_u32(c.ws.route_row + tk);
+    r.w = __uint_as_float(ld_after_wait_u32(weight));
   }
   return r;
 }
-// The row, or kNoSlot. All 32 lanes call.
-__device__ __forceinline__ uint32_t route_place(const SingleCombine& c, const Route& r, uint32_t t) {
-  const bool valid = r.expert < static_cast<uint32_t>(c.cfg.num_experts);
-  if (c.cfg.combine_mode == kCombinePerRoute && (c.recv.external || t < r.dispatched)) return valid ? r.row : kNoSlot;
-  const bool any = __any_sync(0xffffffffu, valid);
-  if (t < r.dispatched) return any ? r.row : kNoSlot;
-  if (any && (threadIdx.x & 31u) == 0) report(c.ws, kStatusWaitTimeout, kPhaseCombineRecv, t, r.dispatched);
+// Tokens that were dispatched: the rows of a later one never come.
+__device__ __forceinline__ uint32_t tokens_dispatched(const SingleCombine& c) {
+  return c.recv.external ? ~0u : ld_after_wait_u32(&c.ws.expert_meta[1]);
+}
+__device__ __noinline__ uint32_t route_of_a_later_token(const A2ALocal& ws, bool valid, uint32_t t, uint32_t dispatched) {
+  if (__any_sync(0xffffffffu, valid) && (threadIdx.x & 31u) == 0) report(ws, kStatusWaitTimeout, kPhaseCombineRecv, t, dispatched);
   return kNoSlot;   // the table holds an earlier dispatch's
+}
+// The row, or kNoSlot. All 32 lanes call.
+__device__ __forceinline__ uint32_t route_place(const SingleCombine& c, const Route& r, uint32_t t, uint32_t dispatched) {
+  bool valid = r.expert < static_cast<uint32_t>(c.cfg.num_experts);
+  if (c.cfg.combine_mode != kCombinePerRoute) valid = __any_sync(0xffffffffu, valid);
+  if (t >= dispatched) return route_of_a_later_token(c.ws, valid, t, dispatched);
+  return valid ? r.row : kNoSlot;
 }
 
 // acc += w_k * row_k over the rows of `have` (bit k: row k is there), 16 bytes of each, at `p` and every
@@ -484,11 +489,6 @@ __global__ void __launch_bounds__(kBulkWarps * 32, 1) combine_bulk_kernel(const 
   const CombineRecvArgs& a = c.recv;
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   const uint32_t K = cfg.topk;
-  grid_wait();
-  grid_allow_next();
-  const uint32_t T = bounded_tokens(cfg, a.num_tokens, a.bound_m);
-  const uint32_t epoch = a.external ? read_epoch(c.ws, 1) : 0u;
-  const uint32_t status = *reinterpret_cast<volatile const uint32_t*>(&c.ws.status[0]);
   uint64_t* const bars = s_bars[warp];
   if (lane == 0) {
     mbar_init(&bars[0], 1);
@@ -496,6 +496,12 @@ __global__ void __launch_bounds__(kBulkWarps * 32, 1) combine_bulk_kernel(const 
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncwarp();
+  grid_wait();
+  grid_allow_next();
+  const uint32_t T = bounded_tokens(cfg, a.num_tokens, a.bound_m);
+  const uint32_t epoch = a.external ? read_epoch(c.ws, 1) : 0u;
+  const uint32_t dispatched = tokens_dispatched(c);
+  const uint32_t status = combine_status(c);
   constexpr int N = VecElems<Y>::N;   // elements of a 16-byte vector
   const uint32_t row_bytes = static_cast<uint32_t>(cfg.hidden_dim) * sizeof(Y);
   const uint32_t seg = c.segment;     // bytes of every row in a piece, a multiple of 512
@@ -506,14 +512,14 @@ __global__ void __launch_bounds__(kBulkWarps * 32, 1) combine_bulk_kernel(const 
   uint32_t job = blockIdx.x * kBulkWarps + warp;   // the warps of a block work on neighbouring pieces
   auto route = [&](uint32_t j) { return j < jobs ? load_route(c, j / pieces, lane) : Route(); };
   const Route first = route(job);
-  if (combine_ready(c, status)) {
+  if (__all_sync(0xffffffffu, status == 0)) {
     // rows of a kernel that is still running on another stream: written by plain stores that the
     // arrival counter covers, read by the bulk-copy engine below
     if (a.external) asm volatile("fence.proxy.async;" ::: "memory");
     uint8_t* const buffers = dyn_smem + warp * 2 * kBulkBuffer;
     auto fetch = [&](uint32_t j, const Route& route, uint32_t slot) -> uint32_t {   // returns which rows come
       if (j >= jobs) return 0;
-      const uint32_t r = route_place(c, route, j / pieces);
+      const uint32_t r = route_place(c, route, j / pieces, dispatched);
       const uint32_t have = __ballot_sync(0xffffffffu, r != kNoSlot);
       if (have != 0) {
         const uint32_t off = j % pieces * seg;
@@ -573,57 +579,50 @@ __global__ void __launch_bounds__(kCombineThreads, 1) combine_single_kernel(cons
   grid_allow_next();
   const int T = bounded_tokens(cfg, a.num_tokens, a.bound_m);
   const uint32_t epoch = a.external ? read_epoch(ws, 1) : 0u;
-  const uint32_t status = *reinterpret_cast<volatile const uint32_t*>(&ws.status[0]);
+  const uint32_t dispatched = tokens_dispatched(c);
+  const uint32_t status = combine_status(c);
   const uint32_t ngran = cfg.hidden_dim / 8;
   const uint32_t pieces = (ngran + 31) / 32;
   constexpr int kVecs = Elem8<Y>::kBytes / 16;
   constexpr int U = 8 / kVecs;   // rows in flight per lane
   const uint32_t warps = gridDim.x * kCombineWarps;
-  const uint32_t first = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-  uint32_t my_row = kNoSlot;   // the first unit's come in with the status word
-  float my_w = 0.f;
-  auto route = [&](uint32_t t) {
-    const Route r = load_route(c, t, lane);
-    my_row = route_place(c, r, t);
-    my_w = r.w;
-  };
-  if (first < T * pieces) route(first / pieces);
-  if (combine_ready(c, status)) {
-    for (uint32_t unit = first; unit < T * pieces; unit += warps) {
-      const uint32_t t = unit / pieces;
-      if (unit != first) route(t);
-      uint8_t* out_row = a.out_tokens + static_cast<uint64_t>(t) * a.out_tokens_stride * sizeof(O);
-      const uint32_t g = unit % pieces * 32 + lane;
-      const bool inside = g < ngran;
-      float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      if (a.accumulate && inside) Elem8<O>::load(out_row + static_cast<uint64_t>(g) * Elem8<O>::kBytes, acc, true);
-      for (uint32_t k0 = 0; k0 < K; k0 += U) {
-        // raw bytes in flight, converted as they are added: as floats they would not fit the registers
-        Vec16 v[U][kVecs];
-        float w[U];
+  for (uint32_t unit = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; unit < T * pieces; unit += warps) {
+    const uint32_t t = unit / pieces;
+    const Route route = load_route(c, t, lane);
+    if (__any_sync(0xffffffffu, status != 0)) break;   // comes in with the first routes
+    const uint32_t my_row = route_place(c, route, t, dispatched);
+    const float my_w = route.w;
+    uint8_t* out_row = a.out_tokens + static_cast<uint64_t>(t) * a.out_tokens_stride * sizeof(O);
+    const uint32_t g = unit % pieces * 32 + lane;
+    const bool inside = g < ngran;
+    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (a.accumulate && inside) Elem8<O>::load(out_row + static_cast<uint64_t>(g) * Elem8<O>::kBytes, acc, true);
+    for (uint32_t k0 = 0; k0 < K; k0 += U) {
+      // raw bytes in flight, converted as they are added: as floats they would not fit the registers
+      Vec16 v[U][kVecs];
+      float w[U];
+      #pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint32_t row = __shfl_sync(0xffffffffu, my_row, k0 + u);
+        w[u] = __shfl_sync(0xffffffffu, my_w, k0 + u);
+        const bool have = inside && k0 + u < K && row != kNoSlot;
+        w[u] = have ? w[u] : 0.f;
+        const uint8_t* p = c.rows + static_cast<uint64_t>(row) * c.row_stride + static_cast<uint64_t>(g) * Elem8<Y>::kBytes;
         #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const uint32_t row = __shfl_sync(0xffffffffu, my_row, k0 + u);
-          w[u] = __shfl_sync(0xffffffffu, my_w, k0 + u);
-          const bool have = inside && k0 + u < K && row != kNoSlot;
-          w[u] = have ? w[u] : 0.f;
-          const uint8_t* p = c.rows + static_cast<uint64_t>(row) * c.row_stride + static_cast<uint64_t>(g) * Elem8<Y>::kBytes;
-          #pragma unroll
-          for (int i = 0; i < kVecs; ++i) v[u][i] = have ? ld_stream_v4(p + 16 * i) : Vec16{0, 0, 0, 0};
-        }
+        for (int i = 0; i < kVecs; ++i) v[u][i] = have ? ld_stream_v4(p + 16 * i) : Vec16{0, 0, 0, 0};
+      }
+      #pragma unroll
+      for (int u = 0; u < U; ++u) {
         #pragma unroll
-        for (int u = 0; u < U; ++u) {
+        for (int i = 0; i < kVecs; ++i) {
+          float f[8];
+          VecElems<Y>::unpack(v[u][i], f);
           #pragma unroll
-          for (int i = 0; i < kVecs; ++i) {
-            float f[8];
-            VecElems<Y>::unpack(v[u][i], f);
-            #pragma unroll
-            for (int q = 0; q < 8 / kVecs; ++q) acc[i * (8 / kVecs) + q] = fmaf(w[u], f[q], acc[i * (8 / kVecs) + q]);
-          }
+          for (int q = 0; q < 8 / kVecs; ++q) acc[i * (8 / kVecs) + q] = fmaf(w[u], f[q], acc[i * (8 / kVecs) + q]);
         }
       }
-      if (inside) Elem8<O>::store(out_row + static_cast<uint64_t>(g) * Elem8<O>::kBytes, acc);
     }
+    if (inside) Elem8<O>::store(out_row + static_cast<uint64_t>(g) * Elem8<O>::kBytes, acc);
   }
   combine_finish(c, epoch);
 }

@@ -40,6 +40,12 @@ __device__ __forceinline__ Vec16 ld_after_wait_v4(const void* p) {
   return v;
 }
 
+__device__ __forceinline__ uint32_t ld_after_wait_u32(const void* p) {
+  uint32_t v;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
 // Data that a peer GPU wrote during this kernel's lifetime and that was made
 // visible through an acquire: coherent (weak) load that skips L1 allocation.
 __device__ __forceinline__ Vec16 ld_stream_v4(const void* p) {
