@@ -848,7 +848,7 @@ void LocalDomain::run_write(const PendingWrite& w, RemoteRegion& rr, std::vector
       a.src_pages = scratch;
       a.dst_pages = scratch + num_pages;
     }
-    // CTAs of the bulk-copy kernel: PPLX_COPY_CTAS overrides the default (a fraction of the SMs)
+    // CTAs of the bulk-copy kernel: PPLX_COPY_CTAS overrides the default (see launch_paged_copy)
     static const int copy_ctas = [] {
       const char* env = std::getenv("PPLX_COPY_CTAS");
       return env != nullptr ? std::atoi(env) : 0;

@@ -253,7 +253,8 @@ void TransferEngine::callback_loop() {
   for (;;) {
     TransferCompletionEntry e;
     // Completions come in bursts, and waking a sleeping thread takes longer than a small copy: poll
-    // for a while after the last one before going to sleep.
+    // for a while after the last one before going to sleep. (Also after each 50 ms of sleep: an idle
+    // engine's thread is busy for 0.4 % of the time.)
     const auto until = std::chrono::steady_clock::now() + kCallbackPoll;
     while (cq_size_.load(std::memory_order_acquire) == 0 && !stopped_.load(std::memory_order_relaxed) &&
            std::chrono::steady_clock::now() < until) {

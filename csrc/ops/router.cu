@@ -1,18 +1,19 @@
 // Stand-alone top-k routing, one warp per token.
 //
 // A round of arg-max per chosen expert (router.cuh) costs two warp reductions and a pass over every
-// lane's registers: with 256 experts and k = 8 about 600 instructions a token, and the issue slots
-// are what a large batch waits for (32,768 tokens: 35 us for 17 MB of logits). Here a token takes
-// about half of that, whatever k is:
-//   1. every lane takes the maximum of its own PER_LANE keys;
-//   2. a bound t that at least k of these 32 maxima reach, and only a few more, is found by bisection
+// lane's registers, and the issue slots are what a large batch waits for: 32,768 tokens of 256 experts
+// with k = 8 took 36 us for 17 MB of bf16 logits, and take 21 us (507 warp instructions a token) here,
+// nearly whatever k is:
+//   1. every lane takes the maximum of its own keys;
+//   2. a bound t that at least k of these maxima reach, and only a few more, is found by bisection
 //      (a comparison, a ballot and a count a step); the k-th largest key is no smaller;
 //   3. the keys >= t, usually k and a few more, are compacted into shared memory, one per lane;
 //   4. a candidate's rank among them is its place in the result.
-// Ties break to the lower expert index, which is part of the comparison. More than 32 candidates need
-// many logits tied with the bound; such a token takes the rounds of router.cuh.
+// Ties break to the lower expert index, which is part of the comparison. With more than 32 candidates (many
+// logits tied with the bound, or a large k) a token takes the rounds of router.cuh; where that is the
+// rule, and where k is 1 or 2, a kernel that does nothing else runs instead (rounds_win() below).
 // Ranking the maxima against one another instead of the bisection, and carrying the logits along
-// instead of reading the k chosen ones again, took 655 instructions a token and 26.6 us.
+// instead of reading the k chosen ones again, took 26.6 us.
 #include "router.h"
 
 #include <cuda_bf16.h>
@@ -239,7 +240,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32) topk_rounds_kernel(const __gri
 // 256 experts k = 20 73 and 66, k = 24 85 and 102; 320 experts k = 14 102 and 76, k = 16 114 and 130; 512
 // experts k = 18 135 and 87, k = 20 146 and 157; 1000 experts k = 20 335 and 304, k = 24 379 and 428. With four
 // keys a lane or fewer the ranking keeps up at any k (128 experts k = 32 84 and 75). One or two rounds are
-// shorter than the ranking's set-up where a lane holds four or eight keys (256 experts k = 1 16.2 and 17.7).
+// shorter than the ranking's set-up where a lane holds four or eight keys (256 experts k = 1 13.1 and 17.5).
 template <int PER_LANE>
 bool rounds_win(int experts, int k, bool vec) {
   if (k <= 2) return PER_LANE == 4 || PER_LANE == 8;

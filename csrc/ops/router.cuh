@@ -1,6 +1,6 @@
 // Top-k routing of one token by one warp without shared memory: what the all-to-all's dispatch uses
 // when it routes a token in the team that is about to send it, and what the stand-alone kernel
-// (router.cu) falls back to when a token's logits tie too often for its own way.
+// (router.cu) does where its own way has too many candidates or is the longer one.
 //
 // Each lane keeps PER_LANE logits in registers (expert = j * 32 + lane, so the loads of a warp
 // are coalesced). The choice is made on logit + bias, mapped to an unsigned key of the same

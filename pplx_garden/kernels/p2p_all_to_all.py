@@ -314,10 +314,11 @@ class P2PAllToAll(AllToAllKernel):
         logits: Optional[torch.Tensor] = None,
         logits_bias: Optional[torch.Tensor] = None,
     ) -> None:
-        """``logits`` ([tokens, num_experts] fp32 or bf16) fuses the routing into the dispatch: the
-        kernel picks each token's top-k experts on ``logits + logits_bias``, takes the softmax over
+        """``logits`` ([tokens, num_experts] fp32 or bf16) fuses the routing into the dispatch: it
+        picks each token's top-k experts on ``logits + logits_bias``, takes the softmax over
         the chosen logits, WRITES them to ``indices`` / ``weights`` (pass these to ``combine``) and
-        sends by them, all in the team that moves the token."""
+        sends by them, all in the team that moves the token. In a group of one rank, send and receive in
+        one call, the routing is a launch of its own in front of the dispatch's."""
         assert self._all_to_all is not None
         if not _torch_ops.a2a_dispatch(self._plan, out_expert_num_tokens, out_expert_x, out_expert_x_scale, dp_x,
                                        dp_x_scale, indices, weights, bound_m, do_send, do_recv, logits, logits_bias):

@@ -112,8 +112,8 @@ class ExpertParallelMoE:
                 out: Optional[torch.Tensor] = None, logits: Optional[torch.Tensor] = None,
                 logits_bias: Optional[torch.Tensor] = None) -> torch.Tensor:
         """x bf16 [tokens, hidden]; indices uint32 and weights fp32 [tokens, k]. With ``logits``
-        ([tokens, experts]) the routing is made inside the dispatch kernel, which fills ``indices``
-        and ``weights``; without, they are inputs."""
+        ([tokens, experts]) the dispatch routes (inside its kernel; in a group of one rank by a launch of
+        its own) and fills ``indices`` and ``weights``; without, they are inputs."""
         assert x.dtype == torch.bfloat16 and x.shape[1] == self.hidden_dim
         if out is None:
             out = torch.empty_like(x)
