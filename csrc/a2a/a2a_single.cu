@@ -14,7 +14,7 @@
 // Both are bound by HBM at prefill sizes and by the chain index -> row -> bytes at decode sizes. Hidden 7168
 // bf16, top-8 of 256 experts, a pass of both: 4096 tokens 429 us with the general kernels, 191 us here
 // (529 MB each way, 81 us at the measured copy rate; one after another and with cold caches the dispatch
-// takes 100 us, the combine 88); 128 tokens 31 and 13.2 us.
+// takes 100 us, the combine 89); 128 tokens 31 and 13.2 us.
 //
 // The tables that the general combine and the expert GEMM's scatter mode read (row_src, row_tk,
 // expert_meta, rec_*) are filled too, so that any combine may follow. The epoch words are left alone:

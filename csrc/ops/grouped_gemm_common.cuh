@@ -105,9 +105,10 @@ __device__ __forceinline__ void decode_tile(const Schedule& s, int num_experts, 
 
 // Rows of A beyond an expert's end are zeros in shared memory. Any bytes would do for the result (a row of D
 // depends on its own row of A, and these are not stored), but the kernels run at the GPU's power limit,
-// and products with the next expert's tokens draw power that products with zeros do not: an expert
-// layer of 32 x 7168 x 2048 on 97 tokens ran at 1.24 GHz and 297 us, and does at 1.50 GHz and 276 us, and
-// on 4096 tokens (a tile in eight is half empty) 1657 -> 1585 us.
+// and products with the next expert's tokens draw power that products with zeros do not. Timed in turn
+// on one GPU, full boxes and zeros: an expert layer of 32 x 7168 x 2048 on 97 tokens 273 and 261 us (1.24 and
+// 1.50 GHz), the GEMMs of 16384 and 8192 rows on 16 and 8 experts 1 % apart, and the layer on 4096
+// tokens, where a tile row in eight is empty, within the noise of 2 %.
 // A tile's rows are counted in units of 16 and fetched in one copy, by the map whose box has the
 // height that covers them; the rest of a stage is filled with zeros by copies of boxes that lie outside
 // of A, which read no memory, and only where the stage's last use left something else there. Boxes of
