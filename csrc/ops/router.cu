@@ -85,7 +85,7 @@ __device__ __forceinline__ void load_run(const T* p, float (&v)[PER_LANE]) {
 }
 
 template <int PER_LANE>
-__device__ __noinline__ void route_by_rounds(const TopkRouteParams& p, int token, int lane) {
+__device__ __forceinline__ void rounds_of_token(const TopkRouteParams& p, int token, int lane) {
   const void* row = static_cast<const char*>(p.logits) + static_cast<int64_t>(token) * p.logits_stride * (p.logits_bf16 ? 2 : 4);
   uint32_t idx;
   float weight;
@@ -94,6 +94,12 @@ __device__ __noinline__ void route_by_rounds(const TopkRouteParams& p, int token
     p.indices[token * p.indices_stride + lane] = idx;
     p.weights[token * p.weights_stride + lane] = weight;
   }
+}
+
+// As a call: the ranking kernel needs its registers for other things.
+template <int PER_LANE>
+__device__ __noinline__ void route_by_rounds(const TopkRouteParams& p, int token, int lane) {
+  rounds_of_token<PER_LANE>(p, token, lane);
 }
 
 __device__ __forceinline__ float to_float(float x) { return x; }
@@ -221,16 +227,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32) topk_rounds_kernel(const __gri
   grid_allow_next();
   const int tokens = p.bound != nullptr ? min(p.tokens, *p.bound) : p.tokens;
   const int token = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (token >= tokens) return;
-  const int lane = threadIdx.x & 31;
-  uint32_t idx;
-  float weight;
-  route_token_warp<PER_LANE>(static_cast<const char*>(p.logits) + static_cast<int64_t>(token) * p.logits_stride * (p.logits_bf16 ? 2 : 4),
-                             p.logits_bf16, p.bias, p.num_experts, p.k, &idx, &weight);
-  if (lane < p.k) {
-    p.indices[token * p.indices_stride + lane] = idx;
-    p.weights[token * p.weights_stride + lane] = weight;
-  }
+  if (token < tokens) rounds_of_token<PER_LANE>(p, token, threadIdx.x & 31);
 }
 
 // Whether the rounds alone beat the ranking. Its candidates have to fit 32 places: with L lanes that hold
