@@ -115,6 +115,9 @@ def write_ninja(verbose: bool, sanitize: str | None = None) -> Path:
         f"cxx = {os.environ.get('CXX', 'g++')}",
         f"nvcc = {CUDA_HOME}/bin/nvcc",
         f"cxxflags = {' '.join(cxxflags + common_inc)}",
+        # The tokenizer's inner loops run 6 % slower or faster by where they fall in a cache line (10 MB on
+        # eight threads 36.9 and 34.5 ms), and without this that depends on the sizes of the objects linked before.
+        "alignflags = -falign-functions=64 -falign-loops=32",
         f"pyflags = -I{py_inc} -I{_pybind_include()}",
         f"torchflags = -I{py_inc} -isystem {_torch_dir()}/include",
         f"torchlibs = -L{_torch_dir()}/lib -ltorch_python -ltorch_cpu -lc10 -lc10_cuda -Wl,-rpath,{_torch_dir()}/lib",
@@ -175,7 +178,9 @@ def write_ninja(verbose: bool, sanitize: str | None = None) -> Path:
             else:
                 lines.append(f"build {obj}: cxx {src}")
                 if rel.parts[0] == "bindings":
-                    lines.append("  extra = $pyflags")
+                    lines.append("  extra = $pyflags" + (" $alignflags" if rel.stem == "py_unigram" else ""))
+                elif rel.parts[0] == "unigram":
+                    lines.append("  extra = $alignflags")
                 elif rel.parts[0] == "torch_ops":
                     lines.append("  extra = $torchflags")
             objs.append(str(obj))
